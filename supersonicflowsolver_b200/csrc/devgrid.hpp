@@ -7,6 +7,8 @@
 #pragma once
 #include <cstdint>
 
+#include <vector_types.h>
+
 namespace psst {
 
 // Primitive state of a volume: p, T, rho, u0, u1, (u2), padding.
@@ -159,48 +161,55 @@ struct LoopCtl {
     double *hist_linf, *hist_l2;  // [cap_rows][dim+2]
 };
 
-// Wavefront schedule of the sequential LocalAccTime1 (the reference's in-loop
-// order, psstFiniteVolumeGrid.cpp:317-323) over many RK stages in one
-// persistent launch. Cell c's level exceeds the level of every interior
-// neighbour updated before it; D is the largest level difference across an
-// interior face and P = D + 1. Operation m of the call (a gradient or an RK
-// stage) of cell c runs at step P m + level(c): every input it needs -- the
-// previous operation of each neighbour and this operation of each earlier
-// neighbour -- is then at least one step (one grid barrier) old. Work items
-// are chunks (at most one block) of one level; they are ordered by level mod
-// P, then level, so the items of one step are contiguous.
-struct WfSched {
-    int32_t period;          // P
-    int32_t nlevels, nitems;
+// Schedule of the resident launch (resident.cuh). Cells are grouped into items
+// of 32 cells of one level. Parallel modes: one level, period 1. Sequential
+// LocalAccTime1 (the reference's in-loop order, psstFiniteVolumeGrid.cpp:
+// 317-323): a cell's level exceeds that of every interior neighbour updated
+// before it, D is the largest level difference across an interior face and P =
+// D + 1. Operation m (a gradient or an RK stage) of a cell has the place P m +
+// level in the order in which every CTA works: all it needs -- the previous
+// operation of each neighbour and this operation of each earlier neighbour --
+// has an earlier place. Items are numbered by level mod P, then level; CTA b
+// owns the items b, b + CTAs, ..
+struct ResSched {
+    int32_t period;             // P
+    int32_t nitems;
+    int32_t max_turn;           // largest level / P
+    int32_t rounds;             // most rounds of four faces of a cell
+    int32_t smem_items;         // items of a CTA kept in shared memory
     const int32_t *cells32;     // [nitems][32] the cells of each item (-1: empty slot)
-    const uint32_t *lowmask;    // [nint] bit q: the cell across CSR entry q was updated
-                                // before this cell in the reference's order
-    const int32_t *item_level;  // [nitems]
-    const int32_t *lvl_items;   // [2 nlevels] item range [first, end) of each level
-    double *ipart;              // [2][nitems][2 NV] per item: sum res^2, max |res| (by operation parity)
-    double *acc;                // [nacc][2 NV] per RK stage: the same over the levels folded so far
-    int32_t nacc;
-    void *grec2;                // second gradient buffer (gradients by iteration parity)
-    unsigned *sync;             // grid barrier: arrivals, generation, abort flag (one 128-byte line each)
+    const uint4 *faces;         // [nitems][rounds] FaceData blocks: static data per lane
+    const double2 *cells;       // [nitems][32] volume, its reciprocal
+    bool same_order;            // every cell's own face order is the face-loop order
+    bool seq;                   // sequential LocalAccTime1
+    const int32_t *own_ptr;     // [CTAs + 1]
+    const int2 *own;            // per CTA, in working order: item, level / P
+    char *store;                // [nitems] ItemStore of the items not in shared memory
+    double *rows;               // [stages of the call][nitems][2 NV] per item: sum res^2, max |res|
+    unsigned *sync;             // finished CTAs (monotonic), abort flag (one 128-byte line each)
+    unsigned arrive_target;     // value of the count once every CTA of this launch has finished
 };
 
 template <typename R>
-struct WfArgs {
+struct ResArgs {
     DevGrid g;
-    CellRec<R> *buf[2];  // state buffers; a stage reads one and writes the other
+    const CellRec<R> *in;   // the call's input state
+    CellRec<R> *out;        // its result; the ghosts' states throughout
+    uint64_t *state[2];     // published states (Record), by stage parity: [nint]
+    uint64_t *proj;         // published gradient projections: [nitems][rounds][128]
+    uint32_t tag0, ptag0;   // stage s publishes tag tag0 + s + 1, iteration k's gradient ptag0 + k + 1
     DevWork<R> wk;
-    void *gbuf[2];       // gradient buffers of the iterations n-1, n-3, .. ([0]) and n-2, .. ([1])
-    WfSched sc;
+    ResSched sc;
     Gas gas;
-    double cfl;
+    double cfl, dt_uniform, rcv;  // rcv: 1 / cv
     double alpha[16];
-    int32_t nst;      // RK stages per iteration
-    int32_t nopi;     // operations per iteration: nst, + 1 with a gradient
-    int64_t nops;     // operations of the call
+    int32_t nst;         // RK stages per iteration
+    int32_t nopi;        // operations per iteration: nst, + 1 with a gradient
     int32_t n_iter;
-    int32_t flux, grad, celllim;
-    int32_t in_buf;   // buffer holding the call's input state
-    uint64_t wait_ns; // bound of each grid-barrier wait (0: do not wait)
+    int32_t nops;        // operations of the launch
+    int32_t nops_stage;  // RK stages of the launch
+    int32_t flux, grad, celllim, lc;
+    uint64_t wait_ns;    // bound of each wait (0: do not wait)
 };
 
 }  // namespace psst

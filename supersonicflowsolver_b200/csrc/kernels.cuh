@@ -144,40 +144,12 @@ __device__ __forceinline__ T ld16(const T *p) {
     for (int i = 0; i < (int)(sizeof(T) / 16); ++i) u.v[i] = q[i];
     return u.t;
 }
-// ldcg: 128-bit loads through L2 only (ld.global.cg), for records that other
-// CTAs of a persistent launch write between its grid barriers: an L1-cached
-// load could return a line this SM kept from before the write. Volatile, so
-// the compiler neither merges nor hoists it across steps.
-template <typename T>
-__device__ __forceinline__ T ldcg(const T *p) {
-    static_assert(sizeof(T) % 16 == 0, "record size must be a multiple of 16 bytes");
-    union U {
-        T t;
-        uint32_t w[sizeof(T) / 4];
-        __device__ U() {}
-    } u;
-    const char *q = reinterpret_cast<const char *>(p);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(T) / 16); ++i)
-        asm volatile("ld.global.cg.v4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(u.w[4 * i]), "=r"(u.w[4 * i + 1]), "=r"(u.w[4 * i + 2]), "=r"(u.w[4 * i + 3])
-                     : "l"(q + 16 * i));
-    return u.t;
-}
+// ldcg: through L2 only, for values that other CTAs of a persistent launch wrote.
 __device__ __forceinline__ double ldcg(const double *p) {
     double v;
     asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
-// state and gradient records: ldg in the pass kernels, ldcg in the persistent one
-template <bool CG, typename T>
-__device__ __forceinline__ T ldst(const T *p) {
-    if constexpr (CG)
-        return ldcg(p);
-    else
-        return ldg(p);
-}
-
 template <typename T>
 __device__ __forceinline__ void st16(T *p, const T &t) {
     static_assert(sizeof(T) % 16 == 0, "record size must be a multiple of 16 bytes");
@@ -296,51 +268,18 @@ __device__ __forceinline__ void boundary_flux(const Prim<R, DIM> &s, const R nn[
     flow[DIM + 1] = s.rho * vn * H;
 }
 
-// One side of the cell-limited MUSCL reconstruction: phi_f = phi_c +
-// (psi_c grad(phi)_c) . (x_f - x_c), the record holding psi_c grad(phi)_c;
-// rho_f = p_f / (R T_f) as in the DM reconstruction.
-template <typename R, int DIM>
-__device__ __forceinline__ void muscl_side(Prim<R, DIM> &r, const GradRec<R, DIM> &gr, const R off[DIM], R rm) {
+// Face states from the two cells' gradient projections (d0 of neighbour 0's
+// gradients, d1 of neighbour 1's). REC 1: Darwish-Moukalled with limiter LIM
+// (psstReconstructorDM::reconstruct_vals, psstValueReconstructor.cpp:70-134),
+// projections on x_c0 - x_c1. REC 2: cell-limited MUSCL, phi_f = phi_c + (psi_c
+// grad(phi)_c) . (x_f - x_c), projections on each side's x_f - x_c. rho_f =
+// p_f / (R T_f) in both.
+template <typename R, int DIM, int REC, int LIM>
+__device__ __forceinline__ void reconstruct(Prim<R, DIM> r[2], const R d0[DIM + 2], const R d1[DIM + 2], R rm) {
 #pragma unroll
     for (int i = 0; i < DIM + 2; ++i) {
-        R d = (R)0;
-#pragma unroll
-        for (int k = 0; k < DIM; ++k) d += gr.g[i * DIM + k] * off[k];
-        pvar<R, DIM>(r, i) += d;
-    }
-    r.rho = r.p / (rm * r.T);
-}
-
-// Interior face: reconstruction (REC 0 first order, 1 Darwish-Moukalled with
-// limiter LIM, 2 cell-limited MUSCL) and the Riemann flux FLUX (1 AUSM, 2 HLL,
-// 3 HLLC). r[0] is neighbour 0 (c0), r[1] neighbour 1. Returns false when the
-// wave speeds cannot be ordered (the reference throws there).
-template <typename R, int DIM, int FLUX, int REC, int LIM>
-__device__ __forceinline__ bool interior_flux(Prim<R, DIM> r[2], const GradRec<R, DIM> *gr0,
-                                              const GradRec<R, DIM> *gr1, const FaceRec<R, DIM> &fr,
-                                              const R nn[DIM], const Gas &gas, R flow[DIM + 2]) {
-    const R rm = (R)gas.rm;
-    if (REC == 1) {  // psstReconstructorDM::reconstruct_vals (psstValueReconstructor.cpp:70-134)
-        // projections of neighbour 0's gradients first, then neighbour 1's (same
-        // sums), so one gradient record is dead before the other is read
-        R dra[DIM + 2], dla[DIM + 2];
-#pragma unroll
-        for (int i = 0; i < DIM + 2; ++i) {
-            R dr = (R)0;
-#pragma unroll
-            for (int k = 0; k < DIM; ++k) dr += gr0->g[i * DIM + k] * fr.o0[k];
-            dra[i] = dr;
-        }
-#pragma unroll
-        for (int i = 0; i < DIM + 2; ++i) {
-            R dl = (R)0;
-#pragma unroll
-            for (int k = 0; k < DIM; ++k) dl += gr1->g[i * DIM + k] * fr.o0[k];
-            dla[i] = dl;
-        }
-#pragma unroll
-        for (int i = 0; i < DIM + 2; ++i) {
-            const R dl = dla[i], dr = dra[i];
+        if (REC == 1) {
+            const R dl = d1[i], dr = d0[i];
             const R v0 = pvar<R, DIM>(r[0], i), v1 = pvar<R, DIM>(r[1], i);
             const R vlm = v1 - ((R)2 * dl - (v0 - v1));
             const R vlp = v0;
@@ -350,13 +289,33 @@ __device__ __forceinline__ bool interior_flux(Prim<R, DIM> r[2], const GradRec<R
             const R nr = vrm - v0, dnr = v0 - vrp;
             pvar<R, DIM>(r[0], i) += (R)0.5 * limiter_value<LIM, R>(nr, dnr) * dnr;
             pvar<R, DIM>(r[1], i) += (R)0.5 * limiter_value<LIM, R>(nl, dnl) * dnl;
+        } else {
+            pvar<R, DIM>(r[0], i) += d0[i];
+            pvar<R, DIM>(r[1], i) += d1[i];
         }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) r[j].rho = r[j].p / (rm * r[j].T);
-    } else if (REC == 2) {  // cell-limited MUSCL (limiters 4, 5)
-        muscl_side<R, DIM>(r[0], *gr0, fr.o0, rm);
-        muscl_side<R, DIM>(r[1], *gr1, fr.o1, rm);
     }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) r[j].rho = r[j].p / (rm * r[j].T);
+}
+
+// Projections of one cell's gradient record on an offset.
+template <typename R, int DIM>
+__device__ __forceinline__ void project(const GradRec<R, DIM> &gr, const R off[DIM], R d[DIM + 2]) {
+#pragma unroll
+    for (int i = 0; i < DIM + 2; ++i) {
+        d[i] = (R)0;
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) d[i] += gr.g[i * DIM + k] * off[k];
+    }
+}
+
+// Riemann flux FLUX (1 AUSM, 2 HLL, 3 HLLC) of the face states r[0] (neighbour
+// 0, c0), r[1] (neighbour 1). Returns false when the wave speeds cannot be
+// ordered (the reference throws there).
+template <typename R, int DIM, int FLUX>
+__device__ __forceinline__ bool riemann_flux(const Prim<R, DIM> r[2], const R nn[DIM], const Gas &gas,
+                                             R flow[DIM + 2]) {
+    const R rm = (R)gas.rm;
     const R cp = (R)gas.cp, cv = (R)gas.cv, gamma = (R)gas.gamma;
     R vn[2], a[2], H[2], M[2], vsq[2];
 #pragma unroll
@@ -498,6 +457,22 @@ __device__ __forceinline__ bool interior_flux(Prim<R, DIM> r[2], const GradRec<R
     return true;
 }
 
+// Interior face: reconstruction (REC 0 first order) and Riemann flux; one
+// gradient record's projections are formed before the other's, so one record
+// is dead before the next is read.
+template <typename R, int DIM, int FLUX, int REC, int LIM>
+__device__ __forceinline__ bool interior_flux(Prim<R, DIM> r[2], const GradRec<R, DIM> *gr0,
+                                              const GradRec<R, DIM> *gr1, const FaceRec<R, DIM> &fr,
+                                              const R nn[DIM], const Gas &gas, R flow[DIM + 2]) {
+    if (REC) {
+        R d0[DIM + 2], d1[DIM + 2];
+        project<R, DIM>(*gr0, fr.o0, d0);
+        project<R, DIM>(*gr1, REC == 1 ? fr.o0 : fr.o1, d1);
+        reconstruct<R, DIM, REC, LIM>(r, d0, d1, (R)gas.rm);
+    }
+    return riemann_flux<R, DIM, FLUX>(r, nn, gas, flow);
+}
+
 // ---------------------------------------------------------------------------
 // face pass
 // ---------------------------------------------------------------------------
@@ -590,8 +565,7 @@ __global__ void __maxnreg__(PSST_BUDGET(R, REC == 1 ? PSST_FACE_MAXNREG_DM : PSS
 // Venkatakrishnan (AIAA 93-0880) cell limiter:
 // psi = min over faces of phi(Delta+, Delta-), Delta- = grad . (x_f - x_c).
 // Gradient (and cell limiter) of one interior cell c from the state records
-// `rec`, written to out[c]. CG: state loads through L2 only (the persistent
-// wavefront kernel, where other CTAs write the states between its steps).
+// `rec`, written to out[c].
 // FP32 Green-Gauss gradient (and cell limiter) of interior cell c of a mesh
 // with 4 faces per cell, from the per-entry table g.gcoef: the cell's 4
 // values of each component are one 16-byte load (a warp's load covers whole
@@ -759,10 +733,10 @@ __device__ __forceinline__ void gradient_cell_table64(const DevGrid &g, const Ce
     st16(gout + c, out);
 }
 
-template <typename R, int DIM, int GRAD, int CELLLIM, bool CG>
+template <typename R, int DIM, int GRAD, int CELLLIM>
 __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R> *rec, GradRec<R, DIM> *gout,
                                               int32_t c) {
-    if constexpr (GRAD == 1 && !CG) {
+    if constexpr (GRAD == 1) {
         if (g.gcoef) {
             if constexpr (sizeof(R) == 4)
                 gradient_cell_table<DIM, CELLLIM>(g, rec, gout, c);
@@ -776,7 +750,7 @@ __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R>
     // uniform meshes (all tets, all hexes): the CSR range follows from c, one
     // dependent load less
     const int32_t b = g.kuni ? c * g.kuni : g.csr_ptr[c], K = g.kuni ? g.kuni : g.csr_ptr[c + 1] - b;
-    const Prim<R, DIM> own = unpack<R, DIM>(ldst<CG>(rec + c));
+    const Prim<R, DIM> own = unpack<R, DIM>(ldg(rec + c));
     R gr[NVAR][DIM];
 #pragma unroll
     for (int i = 0; i < NVAR; ++i)
@@ -829,7 +803,7 @@ __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R>
         if (u4) {  // software pipeline: the next face's records load while this face is summed
             int32_t en = e4.x;
             FaceRec<R, DIM> frn = ldg(frec + (en >> 1));
-            CellRec<R> recn = ldst<CG>(rec + n4.x);
+            CellRec<R> recn = ldg(rec + n4.x);
             R betan = (R)g.beta[en >> 1];
             for (int32_t q = 0; q < 4; ++q) {
                 const int32_t ent = en;
@@ -839,7 +813,7 @@ __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R>
                 if (q < 3) {
                     en = pick(e4, q + 1);
                     frn = ldg(frec + (en >> 1));
-                    recn = ldst<CG>(rec + pick(n4, q + 1));
+                    recn = ldg(rec + pick(n4, q + 1));
                     betan = (R)g.beta[en >> 1];
                 }
                 face(ent, fr, oth, beta);
@@ -848,7 +822,7 @@ __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R>
 #endif
         for (int32_t q = 0; q < K; ++q) {  // not unrolled: fewer registers, more blocks (measured faster)
             const int32_t ent = u4 ? pick(e4, q) : g.csr_ent[b + q];
-            face(ent, ldg(frec + (ent >> 1)), unpack<R, DIM>(ldst<CG>(rec + (u4 ? pick(n4, q) : g.csr_nb[b + q]))),
+            face(ent, ldg(frec + (ent >> 1)), unpack<R, DIM>(ldg(rec + (u4 ? pick(n4, q) : g.csr_nb[b + q]))),
                  (R)g.beta[ent >> 1]);
         }
     } else {
@@ -861,7 +835,7 @@ __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R>
         for (int32_t j = 0; j < K; ++j) {
             const int32_t slot = b + (int32_t)((perm >> (4 * j)) & 15);
             const int32_t nb = g.csr_nb[slot];
-            const Prim<R, DIM> oth = unpack<R, DIM>(ldst<CG>(rec + nb));
+            const Prim<R, DIM> oth = unpack<R, DIM>(ldg(rec + nb));
             if (CELLLIM)
 #pragma unroll
                 for (int i = 0; i < NVAR; ++i) {
@@ -940,7 +914,7 @@ __global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_GRAD_MINB, 1)) k_grad
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.nint) return;
     if (g.cell_case && !g.case_active[g.cell_case[c]]) return;  // stopped case
-    gradient_cell<R, DIM, GRAD, CELLLIM, false>(g, st.rec, reinterpret_cast<GradRec<R, DIM> *>(wk.grec), c);
+    gradient_cell<R, DIM, GRAD, CELLLIM>(g, st.rec, reinterpret_cast<GradRec<R, DIM> *>(wk.grec), c);
 }
 
 // cell update
@@ -948,9 +922,8 @@ __global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_GRAD_MINB, 1)) k_grad
 
 // Local time step of one cell (psstLocalTimeCalculation.cpp:90-131, 175-213),
 // faces in the cell's own order. In the sequential mode, neighbours updated
-// earlier in the reference's order are read from `nxt`. CG: neighbour states
-// through L2 only (the persistent wavefront kernel).
-template <typename R, int DIM, int LC, bool SEQ, bool CG = false>
+// earlier in the reference's order are read from `nxt`.
+template <typename R, int DIM, int LC, bool SEQ>
 __device__ __forceinline__ double local_time(const DevGrid &g, const CellRec<R> *cur, const CellRec<R> *nxt,
                                              const Gas &gas, double cfl, double dt_uniform, int32_t c,
                                              const Prim<R, DIM> &own) {
@@ -970,7 +943,7 @@ __device__ __forceinline__ double local_time(const DevGrid &g, const CellRec<R> 
             const FaceRec<R, DIM> fr = ld16(frec + (ent >> 1));
             const int32_t nb = (ent & 1) ? fr.c0 : fr.c1;
             const CellRec<R> *src = (SEQ && nb < g.nint && g.rank[nb] < myrank) ? nxt : cur;
-            const Prim<R, DIM> o = unpack<R, DIM>(CG ? ldcg(src + nb) : ld16(src + nb));
+            const Prim<R, DIM> o = unpack<R, DIM>(ld16(src + nb));
             const R cn = (sqrt(gr * o.T) + cc) * (R)0.5;
             R nv = (R)0;
 #pragma unroll
@@ -1070,22 +1043,19 @@ __device__ __forceinline__ CellRec<R> rk_update(const DevGrid &g, const DevWork<
 // 351-366): dynamic condition (psstBoundaryCondition.cpp:26-37, 72-80, 108-127,
 // 212-219), thermal condition (:285-288, 354-357), rho = p/(T*rm).
 template <typename R, int DIM>
-__device__ __forceinline__ CellRec<R> ghost_state(const DevGrid &g, const CellRec<R> &gcur, const Prim<R, DIM> &nb,
-                                                  int32_t i, const Gas &gas) {
+__device__ __forceinline__ CellRec<R> ghost_from(const CellRec<R> &gcur, const Prim<R, DIM> &nb, int dyn, int th,
+                                                 const R *n, const Gas &gas) {
     Prim<R, DIM> s = unpack<R, DIM>(gcur);
-    const int32_t z = g.g_zone[i];
-    const int dyn = g.z_dyn[z], th = g.z_therm[z];
     if (dyn == 26) {
 #pragma unroll
         for (int k = 0; k < DIM; ++k) s.u[k] = nb.u[k];
         s.p = nb.p;
     } else if (dyn == 15) {
-        const FaceRec<R, DIM> fr = ldg(reinterpret_cast<const FaceRec<R, DIM> *>(g.frec) + g.g_face[i]);
         R vn = (R)0;
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) vn += nb.u[k] * (R)fr.n[k];
+        for (int k = 0; k < DIM; ++k) vn += nb.u[k] * n[k];
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) s.u[k] = nb.u[k] - vn * (R)fr.n[k];
+        for (int k = 0; k < DIM; ++k) s.u[k] = nb.u[k] - vn * n[k];
         s.p = nb.p;
     } else if (dyn == 25) {
 #pragma unroll
@@ -1093,6 +1063,21 @@ __device__ __forceinline__ CellRec<R> ghost_state(const DevGrid &g, const CellRe
     }
     if (th == 25 || th == 18) s.T = nb.T;
     return pack<R, DIM>(s.p, s.T, s.p / (s.T * (R)gas.rm), s.u);
+}
+template <typename R, int DIM>
+__device__ __forceinline__ CellRec<R> ghost_state(const DevGrid &g, const CellRec<R> &gcur, const Prim<R, DIM> &nb,
+                                                  int32_t i, const Gas &gas) {
+    const int32_t z = g.g_zone[i];
+    const int dyn = g.z_dyn[z];
+    R n[DIM];
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) n[k] = (R)0;
+    if (dyn == 15) {  // the wall's normal
+        const FaceRec<R, DIM> fr = ldg(reinterpret_cast<const FaceRec<R, DIM> *>(g.frec) + g.g_face[i]);
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) n[k] = (R)fr.n[k];
+    }
+    return ghost_from<R, DIM>(gcur, nb, dyn, g.z_therm[z], n, gas);
 }
 
 // Block partials of the residual norms: part[block][v] = sum res^2,

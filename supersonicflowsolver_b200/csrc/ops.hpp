@@ -11,9 +11,10 @@ namespace psst {
 
 constexpr int kBlock = 256;
 constexpr int kMinBlock = 64;  // smallest launch shape the tuner may pick
-constexpr int kWfBlock = 128;  // threads per CTA of k_wavefront
-constexpr int kWfLanes = 4;    // lanes per cell in k_wavefront's RK stages (cells per work item: 32)
-constexpr int kWfSyncWords = 96;  // k_wavefront's grid-barrier words (three 128-byte lines)
+constexpr int kWfBlock = 128;  // threads per CTA of k_resident
+constexpr int kWfLanes = 4;    // lanes per cell in k_resident (cells per work item: 32)
+
+constexpr int kWfSyncWords = 96;  // k_resident's counter and flag words (three 128-byte lines)
 constexpr int kNormReduceBlocks = 296;  // blocks of k_norm_reduce (first level of its two-level sum): two per SM
 inline int nblocks(int64_t n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
@@ -69,11 +70,24 @@ struct Ops {
     // iteration count and the while-loop condition `h`
     static void loop_control(int dim, const DevGrid &g, const DevWork<R> &wk, const CaseStop &cs, LoopCtl *ctl,
                              int chunk, cudaGraphConditionalHandle h, cudaStream_t s);
-    // Sequential LocalAccTime1 over a whole call as one cooperative launch of
-    // nblocks CTAs (k_wavefront; FP64 only, cudaErrorNotSupported otherwise).
-    static cudaError_t wavefront(int dim, int rec, int lim, const WfArgs<R> &a, int nblocks, cudaStream_t s);
-    // co-resident CTAs of that kernel on the current device (0: not built)
-    static int wavefront_max_blocks(int dim, int rec, int lim);
+    // A whole call as one cooperative launch of nblocks CTAs (k_resident).
+    static cudaError_t resident(int dim, int rec, int lim, const ResArgs<R> &a, int nblocks, size_t smem,
+                                cudaStream_t s);
+    // co-resident CTAs of that kernel on the current device, with up to `want`
+    // items of a CTA in shared memory (*items of them, *smem bytes)
+    static int resident_max_blocks(int dim, int rec, int lim, int rounds, int want, int *items, size_t *smem);
+    static size_t resident_store_bytes(int dim, int rec, int rounds);  // ItemStore of one item
+    // sizes of its tables and buffers for nint cells in nitems items
+    struct ResidentBytes {
+        size_t lanes, state, proj;
+    };
+    static ResidentBytes resident_bytes(int dim, int64_t nint, int64_t nitems, int rounds);
+    // the static face data of its items (FaceData), from the grid's arrays: mate
+    // per CSR entry the same face's entry in the cell across, pos per cell its
+    // place item * 32 + slot
+    static void resident_build(int dim, int rec, int grad, const DevGrid &g, const int32_t *cells32,
+                               const uint32_t *lowmask, const int32_t *mate, const int32_t *pos, int nitems,
+                               int rounds, void *faces, void *cells, cudaStream_t s);
 };
 
 }  // namespace psst

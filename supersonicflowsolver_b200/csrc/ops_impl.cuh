@@ -5,7 +5,7 @@
 
 #include "kernels.cuh"
 #include "ops.hpp"
-#include "wavefront.cuh"
+#include "resident.cuh"
 
 namespace psst {
 
@@ -279,42 +279,58 @@ void Ops<R>::loop_control(int dim, const DevGrid &g, const DevWork<R> &wk, const
         k_loop_control<5><<<1, kBlock, 0, s>>>(cs, g.ncase, wk.err, ctl, wk.linf, wk.l2, chunk, h);
 }
 
-// ---- sequential LocalAccTime1 as one persistent launch (FP64 only) ----
+// ---- a whole call as one persistent launch ----
 template <typename R, int DIM>
-static cudaError_t wavefront_d(int rec, int lim, const WfArgs<R> &a, int nb, cudaStream_t s) {
-    if (rec == 0) return wf_launch<R, DIM, 0, 1>(a, nb, s);
-    if (rec == 2) return wf_launch<R, DIM, 2, 1>(a, nb, s);
-    if (lim == 1) return wf_launch<R, DIM, 1, 1>(a, nb, s);
-    if (lim == 2) return wf_launch<R, DIM, 1, 2>(a, nb, s);
-    return wf_launch<R, DIM, 1, 3>(a, nb, s);
+static cudaError_t resident_d(int rec, int lim, const ResArgs<R> &a, int nb, size_t smem, cudaStream_t s) {
+    if (rec == 0) return res_launch<R, DIM, 0, 1>(a, nb, smem, s);
+    if (rec == 2) return res_launch<R, DIM, 2, 1>(a, nb, smem, s);
+    if (lim == 1) return res_launch<R, DIM, 1, 1>(a, nb, smem, s);
+    if (lim == 2) return res_launch<R, DIM, 1, 2>(a, nb, smem, s);
+    return res_launch<R, DIM, 1, 3>(a, nb, smem, s);
 }
 template <typename R, int DIM>
-static int wavefront_max_d(int rec, int lim) {
-    if (rec == 0) return wf_max_blocks<R, DIM, 0, 1>();
-    if (rec == 2) return wf_max_blocks<R, DIM, 2, 1>();
-    if (lim == 1) return wf_max_blocks<R, DIM, 1, 1>();
-    if (lim == 2) return wf_max_blocks<R, DIM, 1, 2>();
-    return wf_max_blocks<R, DIM, 1, 3>();
+static int resident_max_d(int rec, int lim, int rounds, int want, int *items, size_t *smem) {
+    if (rec == 0) return res_max_blocks<R, DIM, 0, 1>(rounds, want, items, smem);
+    if (rec == 2) return res_max_blocks<R, DIM, 2, 1>(rounds, want, items, smem);
+    if (lim == 1) return res_max_blocks<R, DIM, 1, 1>(rounds, want, items, smem);
+    if (lim == 2) return res_max_blocks<R, DIM, 1, 2>(rounds, want, items, smem);
+    return res_max_blocks<R, DIM, 1, 3>(rounds, want, items, smem);
 }
 
 template <typename R>
-cudaError_t Ops<R>::wavefront(int dim, int rec, int lim, const WfArgs<R> &a, int nb, cudaStream_t s) {
-    if constexpr (sizeof(R) == 8) {
-        return dim == 2 ? wavefront_d<R, 2>(rec, lim, a, nb, s) : wavefront_d<R, 3>(rec, lim, a, nb, s);
-    } else {
-        (void)dim, (void)rec, (void)lim, (void)a, (void)nb, (void)s;
-        return cudaErrorNotSupported;
-    }
+cudaError_t Ops<R>::resident(int dim, int rec, int lim, const ResArgs<R> &a, int nb, size_t smem, cudaStream_t s) {
+    return dim == 2 ? resident_d<R, 2>(rec, lim, a, nb, smem, s) : resident_d<R, 3>(rec, lim, a, nb, smem, s);
 }
 
 template <typename R>
-int Ops<R>::wavefront_max_blocks(int dim, int rec, int lim) {
-    if constexpr (sizeof(R) == 8) {
-        return dim == 2 ? wavefront_max_d<R, 2>(rec, lim) : wavefront_max_d<R, 3>(rec, lim);
-    } else {
-        (void)dim, (void)rec, (void)lim;
-        return 0;
-    }
+int Ops<R>::resident_max_blocks(int dim, int rec, int lim, int rounds, int want, int *items, size_t *smem) {
+    return dim == 2 ? resident_max_d<R, 2>(rec, lim, rounds, want, items, smem)
+                    : resident_max_d<R, 3>(rec, lim, rounds, want, items, smem);
+}
+
+template <typename R>
+size_t Ops<R>::resident_store_bytes(int dim, int rec, int rounds) {
+    return dim == 2 ? ItemStore<R, 2>::bytes(rounds, rec != 0) : ItemStore<R, 3>::bytes(rounds, rec != 0);
+}
+
+template <typename R>
+typename Ops<R>::ResidentBytes Ops<R>::resident_bytes(int dim, int64_t nint, int64_t nitems, int rounds) {
+    const int pieces = dim == 2 ? FaceData<R, 2>::PIECES : FaceData<R, 3>::PIECES;
+    const int64_t lanes = nitems * rounds * kWfBlock;
+    return ResidentBytes{(size_t)(lanes * pieces * 16), (size_t)(nint * record_words<R>(dim + 3)) * 8,
+                         (size_t)(lanes * record_words<R>(dim + 2)) * 8};
+}
+
+template <typename R>
+void Ops<R>::resident_build(int dim, int rec, int grad, const DevGrid &g, const int32_t *cells32,
+                            const uint32_t *lowmask, const int32_t *mate, const int32_t *pos, int nitems, int rounds,
+                            void *lanes, void *cells, cudaStream_t s) {
+    if (dim == 2)
+        k_res_build<R, 2><<<nitems * rounds, kWfBlock, 0, s>>>(g, rec, grad, cells32, lowmask, mate, pos, rounds,
+                                                               (uint4 *)lanes, (double2 *)cells);
+    else
+        k_res_build<R, 3><<<nitems * rounds, kWfBlock, 0, s>>>(g, rec, grad, cells32, lowmask, mate, pos, rounds,
+                                                               (uint4 *)lanes, (double2 *)cells);
 }
 
 }  // namespace psst

@@ -76,13 +76,21 @@ struct Layout {
     std::vector<int32_t> dev_of_vol;  // reference volume -> device cell (-1: inactive)
     std::vector<int64_t> vol_of_dev;  // device cell -> reference volume
     std::vector<int32_t> c0, c1, csr_ptr, csr_ent, csr_nb, rank, gptr, g_nb, g_face, g_zone, z_dyn, z_therm, lvl_cells, lvl_ptr;
-    // wavefront schedule of the sequential LocalAccTime1 (WfSched)
-    int32_t wf_period = 1, wf_max_class_items = 0;
-    std::vector<int32_t> wf_cells32, wf_item_level, wf_lvl_items;
-    std::vector<uint32_t> wf_lowmask;
+    // schedule of the resident launch (ResSched)
+    int32_t res_period = 1;
+    std::vector<int32_t> res_cells32, res_item_level;
+    std::vector<uint32_t> res_lowmask;
     std::vector<uint64_t> wperm;
     std::vector<double> S, n, xf, beta, V, xc, lsq_r, vk_eps2, z_u, z_p, z_T;
 };
+
+std::vector<int32_t> cell_levels(const Layout &L, int32_t &nlevels);
+void build_resident_items(Layout &L, const std::vector<int32_t> &level, bool seq);
+
+// Most cells for which the parallel modes run as one resident launch: beyond
+// it every CTA has several items to work through per operation, and the pass
+// kernels, which form each interior face's flux once, are faster.
+constexpr int32_t kResidentMaxCells = 40000;
 
 void build_layout(const psst_grid &G, const psst_scheme &sc, Layout &L) {
     const int dim = G.dim;
@@ -316,71 +324,91 @@ void build_layout(const psst_grid &G, const psst_scheme &sc, Layout &L) {
         const double kh = sc.venkat_k * h;
         L.vk_eps2[d] = kh * kh * kh;
     }
-    // level schedule for the sequential LocalAccTime1: a cell's level exceeds
-    // that of every interior neighbour updated before it in the reference.
-    std::vector<int32_t> level(L.nint, 0);
-    std::vector<int32_t> dev_by_rank(L.nint);
+    if (!(sc.lc == 1 && sc.lc1_mode == PSST_LC1_SEQUENTIAL)) {  // nothing walks the levels
+        if (L.nint <= kResidentMaxCells && G.case_vol_ptr.empty()) build_resident_items(L, {}, false);
+        L.lvl_ptr.assign(1, 0);
+        return;
+    }
+    const std::vector<int32_t> level = cell_levels(L, L.nlevels);
+    L.lvl_ptr.assign(L.nlevels + 1, 0);
+    for (int32_t d = 0; d < L.nint; ++d) L.lvl_ptr[level[d] + 1]++;
+    for (int32_t l = 0; l < L.nlevels; ++l) L.lvl_ptr[l + 1] += L.lvl_ptr[l];
+    L.lvl_cells.resize(L.nint);
+    std::vector<int32_t> fillp(L.lvl_ptr.begin(), L.lvl_ptr.end() - 1), dev_by_rank(L.nint);
+    for (int32_t d = 0; d < L.nint; ++d) dev_by_rank[L.rank[d]] = d;
+    for (int32_t r = 0; r < L.nint; ++r) {
+        const int32_t d = dev_by_rank[r];
+        L.lvl_cells[fillp[level[d]]++] = d;
+    }
+    if (L.nint > 0) build_resident_items(L, level, true);
+}
+
+// Level schedule of the sequential LocalAccTime1: a cell's level exceeds that of
+// every interior neighbour updated before it in the reference.
+std::vector<int32_t> cell_levels(const Layout &L, int32_t &nlevels) {
+    std::vector<int32_t> level(L.nint, 0), dev_by_rank(L.nint);
     for (int32_t d = 0; d < L.nint; ++d) dev_by_rank[L.rank[d]] = d;
     int32_t maxlvl = -1;
     for (int32_t r = 0; r < L.nint; ++r) {
         const int32_t d = dev_by_rank[r];
         int32_t lv = 0;
         for (int32_t q = L.csr_ptr[d]; q < L.csr_ptr[d + 1]; ++q) {
-            const int32_t f = L.csr_ent[q] >> 1;
-            const int32_t nb = (L.csr_ent[q] & 1) ? L.c0[f] : L.c1[f];
+            const int32_t nb = L.csr_nb[q];
             if (nb < L.nint && L.rank[nb] < r) lv = std::max(lv, level[nb] + 1);
         }
         level[d] = lv;
         maxlvl = std::max(maxlvl, lv);
     }
-    L.nlevels = maxlvl + 1;
-    L.lvl_ptr.assign(L.nlevels + 1, 0);
-    for (int32_t d = 0; d < L.nint; ++d) L.lvl_ptr[level[d] + 1]++;
-    for (int32_t l = 0; l < L.nlevels; ++l) L.lvl_ptr[l + 1] += L.lvl_ptr[l];
-    L.lvl_cells.resize(L.nint);
-    std::vector<int32_t> fillp(L.lvl_ptr.begin(), L.lvl_ptr.end() - 1);
-    for (int32_t r = 0; r < L.nint; ++r) {
-        const int32_t d = dev_by_rank[r];
-        L.lvl_cells[fillp[level[d]]++] = d;
-    }
-    // wavefront schedule: period P = 1 + the largest level difference across
-    // an interior face; items of at most kWfBlock / kWfLanes cells of one level (device
-    // order inside a level), ordered by level mod P, then level
-    if (sc.lc == 1 && sc.lc1_mode == PSST_LC1_SEQUENTIAL && L.nint > 0) {
-        int32_t D = 0;
-        for (int32_t d = 0; d < L.nint; ++d)
-            for (int32_t q = L.csr_ptr[d]; q < L.csr_ptr[d + 1]; ++q) {
-                const int32_t nb = L.csr_nb[q];
-                if (nb < L.nint) D = std::max(D, std::abs(level[d] - level[nb]));
-            }
-        L.wf_period = D + 1;
-        std::vector<int32_t> by_level(L.nint), fill(L.lvl_ptr.begin(), L.lvl_ptr.end() - 1);
-        for (int32_t d = 0; d < L.nint; ++d) by_level[fill[level[d]]++] = d;
-        L.wf_lvl_items.assign((size_t)2 * L.nlevels, 0);
-        L.wf_cells32.clear();
-        L.wf_item_level.clear();
-        const int32_t per_item = kWfBlock / kWfLanes;
-        for (int32_t r = 0; r < L.wf_period; ++r) {
-            const int32_t first = (int32_t)L.wf_item_level.size();
-            for (int32_t l = r; l < L.nlevels; l += L.wf_period) {
-                L.wf_lvl_items[2 * (size_t)l] = (int32_t)L.wf_item_level.size();
-                for (int32_t b = L.lvl_ptr[l]; b < L.lvl_ptr[l + 1]; b += per_item) {
-                    L.wf_item_level.push_back(l);
-                    for (int32_t i = b; i < b + per_item; ++i)
-                        L.wf_cells32.push_back(i < L.lvl_ptr[l + 1] ? by_level[i] : -1);
-                }
-                L.wf_lvl_items[2 * (size_t)l + 1] = (int32_t)L.wf_item_level.size();
-            }
-            L.wf_max_class_items = std::max(L.wf_max_class_items, (int32_t)L.wf_item_level.size() - first);
+    nlevels = maxlvl + 1;
+    return level;
+}
+
+// Items of the resident launch (ResSched): 32 cells of one level each (device
+// order inside a level), ordered by level mod P, then level; P = 1 + the
+// largest level difference across an interior face. Without the sequential
+// time step all cells are of one level.
+void build_resident_items(Layout &L, const std::vector<int32_t> &level, bool seq) {
+    constexpr int32_t per_item = kWfBlock / kWfLanes;
+    L.res_cells32.clear();
+    L.res_item_level.clear();
+    if (!seq) {
+        for (int32_t b = 0; b < L.nint; b += per_item) {
+            L.res_item_level.push_back(0);
+            for (int32_t i = b; i < b + per_item; ++i) L.res_cells32.push_back(i < L.nint ? i : -1);
         }
-        // neighbours updated before each cell in the reference's order, per CSR entry
-        L.wf_lowmask.assign(L.nint, 0u);
-        for (int32_t d = 0; d < L.nint; ++d)
-            for (int32_t q = L.csr_ptr[d]; q < L.csr_ptr[d + 1]; ++q) {
-                const int32_t nb = L.csr_nb[q];
-                if (nb < L.nint && L.rank[nb] < L.rank[d]) L.wf_lowmask[d] |= 1u << (q - L.csr_ptr[d]);
-            }
+        return;
     }
+    int32_t D = 0;
+    for (int32_t d = 0; d < L.nint; ++d)
+        for (int32_t q = L.csr_ptr[d]; q < L.csr_ptr[d + 1]; ++q) {
+            const int32_t nb = L.csr_nb[q];
+            if (nb < L.nint) D = std::max(D, std::abs(level[d] - level[nb]));
+        }
+    L.res_period = D + 1;
+    std::vector<int32_t> by_level(L.nint), fill(L.lvl_ptr.begin(), L.lvl_ptr.end() - 1);
+    for (int32_t d = 0; d < L.nint; ++d) by_level[fill[level[d]]++] = d;
+    for (int32_t r = 0; r < L.res_period; ++r)
+        for (int32_t l = r; l < L.nlevels; l += L.res_period)
+            for (int32_t b = L.lvl_ptr[l]; b < L.lvl_ptr[l + 1]; b += per_item) {
+                L.res_item_level.push_back(l);
+                for (int32_t i = b; i < b + per_item; ++i)
+                    L.res_cells32.push_back(i < L.lvl_ptr[l + 1] ? by_level[i] : -1);
+            }
+    // neighbours updated before each cell in the reference's order, per CSR entry
+    L.res_lowmask.assign(L.nint, 0u);
+    for (int32_t d = 0; d < L.nint; ++d)
+        for (int32_t q = L.csr_ptr[d]; q < L.csr_ptr[d + 1]; ++q) {
+            const int32_t nb = L.csr_nb[q];
+            if (nb < L.nint && L.rank[nb] < L.rank[d]) L.res_lowmask[d] |= 1u << (q - L.csr_ptr[d]);
+        }
+}
+
+// Per CSR entry, the same face's entry in the cell across (-1: boundary face).
+std::vector<int32_t> mate_entries(const Layout &L) {
+    std::vector<int32_t> at((size_t)2 * L.nface, -1), mate(L.csr_ent.size(), -1);
+    for (size_t q = 0; q < L.csr_ent.size(); ++q) at[(size_t)L.csr_ent[q]] = (int32_t)q;
+    for (size_t q = 0; q < L.csr_ent.size(); ++q) mate[q] = at[(size_t)(L.csr_ent[q] ^ 1)];
+    return mate;
 }
 
 
@@ -502,12 +530,15 @@ struct psst_solver {
     LoopCtl *loopctl = nullptr;
     double *hist_linf = nullptr, *hist_l2 = nullptr;
     int64_t hist_rows = 0;
-    // sequential LocalAccTime1 as one persistent launch per call (FP64, single
-    // grids): schedule uploaded (wf_ready), switched on (wf_on), CTAs, and the
-    // bound of every grid-barrier wait
-    bool wf_ready = false, wf_on = true;
-    WfSched wf{};
-    int wf_blocks = 0;
+    // whole calls as one persistent launch (ResSched): built (res_ready),
+    // switched on (res_on), CTAs, dynamic shared memory, the tags used so far
+    bool res_ready = false, res_on = true, res_dirty = false;
+    ResSched res{};
+    int res_blocks = 0;
+    size_t res_smem = 0;
+    void *res_state[2] = {nullptr, nullptr}, *res_proj = nullptr;
+    size_t res_state_bytes = 0, res_proj_bytes = 0, res_rows_cap = 0;
+    uint32_t res_tag = 0, res_ptag = 0, res_arrived = 0;
     uint64_t wait_ns = kDefaultWaitNs;
     static constexpr uint64_t kDefaultWaitNs = 10000000000ull;  // 10 s; a step takes microseconds
 
@@ -666,7 +697,8 @@ void raise_err(psst_solver *s, const int32_t e[4], const int32_t *err_dev) {
     case 3:
         raise(PSST_ERR_NONFINITE, "non-finite residual in cell " + std::to_string(s->L.vol_of_dev[e[1]]));
     case 5:
-        raise(PSST_ERR_TIMEOUT, "a grid-barrier wait of the wavefront launch ran out (step " + std::to_string(e[1]) +
+        s->res_dirty = true;
+        raise(PSST_ERR_TIMEOUT, "a wait of the resident launch ran out (operation " + std::to_string(e[1]) +
                                     "); the state is undefined until the next psst_solver_set_state");
     default:
         raise(PSST_ERR_NONFINITE, "non-positive density or temperature in cell " + std::to_string(s->L.vol_of_dev[e[1]]));
@@ -718,45 +750,150 @@ void one_stage(psst_solver *s, int k, int it_slot, bool gather, Mark &&mark) {
     s->cur ^= 1;
 }
 
-bool wavefront_active(const psst_solver *s) { return s->seq && s->wf_ready && s->wf_on; }
+bool resident_active(const psst_solver *s) { return s->res_ready && s->res_on; }
 
-// The whole call as one cooperative launch (the wavefront schedule, WfSched);
-// the norm buffers are reserved and zeroed by the caller.
+// Bytes of norm rows that one resident launch may write; a longer call is cut
+// into several launches.
+constexpr size_t kResRowsMax = (size_t)256 << 20;
+
+// Tables and buffers of the resident launch, if the kernel fits the device.
 template <typename R>
-void wavefront_run(psst_solver *s, int n_iter) {
+void build_resident(psst_solver *s) {
+    const Layout &L = s->L;
+    const int32_t nitems = (int32_t)L.res_item_level.size();
+    if (nitems == 0) return;
+    ResSched &w = s->res;
+    int maxk = 1;
+    for (int32_t d = 0; d < L.nint; ++d) maxk = std::max(maxk, L.csr_ptr[d + 1] - L.csr_ptr[d]);
+    w.rounds = (maxk + 3) / 4;
+    int items = 0;
+    const int maxb = Ops<R>::resident_max_blocks(s->dim, s->rec, s->sc.limiter, w.rounds, 2, &items, &s->res_smem);
+    if (maxb <= 0) return;
+    s->res_blocks = std::min(nitems, maxb);
+    w.period = L.res_period;
+    w.seq = s->seq;
+    w.same_order = true;
+    for (int32_t d = 0; d < L.nint && w.same_order; ++d) {
+        const int kd = L.csr_ptr[d + 1] - L.csr_ptr[d];
+        w.same_order = L.wperm[d] == (0xFEDCBA9876543210ull & (kd >= 16 ? ~0ull : (1ull << (4 * kd)) - 1));
+    }
+    w.nitems = nitems;
+    w.smem_items = items;
+    std::vector<int32_t> ptr(1, 0);
+    std::vector<int2> own;
+    int most = 0;
+    for (int b = 0; b < s->res_blocks; ++b) {
+        for (int32_t i = b; i < nitems; i += s->res_blocks) {
+            const int32_t turn = L.res_item_level[i] / L.res_period;
+            own.push_back(int2{i, turn});
+            w.max_turn = std::max(w.max_turn, turn);
+        }
+        most = std::max(most, (int)own.size() - ptr.back());
+        ptr.push_back((int32_t)own.size());
+    }
+    w.own_ptr = s->upload(ptr);
+    w.own = s->upload(own);
+    w.cells32 = s->upload(L.res_cells32);
+    if (most > items)
+        w.store = (char *)s->dalloc_bytes(nitems * Ops<R>::resident_store_bytes(s->dim, s->rec, w.rounds));
+    w.sync = s->dalloc<unsigned>(kWfSyncWords);
+    const auto bytes = Ops<R>::resident_bytes(s->dim, L.nint, nitems, w.rounds);
+    s->res_state_bytes = bytes.state;
+    for (auto &p : s->res_state) p = s->dalloc_bytes(bytes.state);
+    if (s->sc.order == 2) {
+        s->res_proj_bytes = bytes.proj;
+        s->res_proj = s->dalloc_bytes(bytes.proj);
+    }
+    // static lane data, from arrays that only its construction needs
+    std::vector<int32_t> pos(L.nint);
+    for (size_t i = 0; i < L.res_cells32.size(); ++i)
+        if (L.res_cells32[i] >= 0) pos[L.res_cells32[i]] = (int32_t)i;
+    void *lanes = s->dalloc_bytes(bytes.lanes), *cells = s->dalloc_bytes((size_t)nitems * 32 * 2 * sizeof(double));
+    int32_t *d_mate = s->upload(mate_entries(L)), *d_pos = s->upload(pos);
+    uint32_t *d_low = L.res_lowmask.empty() ? nullptr : s->upload(L.res_lowmask);
+    Ops<R>::resident_build(s->dim, s->rec, s->sc.order == 2 ? s->sc.grad : 0, s->g, w.cells32, d_low, d_mate, d_pos,
+                           nitems, w.rounds, lanes, cells, s->stream);
+    ck(cudaGetLastError(), "resident tables");
+    ck(cudaStreamSynchronize(s->stream), "resident tables");
+    s->dfree(d_mate);
+    s->dfree(d_pos);
+    s->dfree(d_low);
+    w.faces = (const uint4 *)lanes;
+    w.cells = (const double2 *)cells;
+    s->res_dirty = true;  // tags cleared before the first launch
+    s->res_ready = true;
+}
+
+// n_iter iterations as cooperative launches of the resident kernel (one,
+// unless the norm rows of the call exceed kResRowsMax).
+template <typename R, typename Mark>
+void resident_run(psst_solver *s, int n_iter, Mark &&mark) {
     DevState<R> *st = states<R>(s);
-    DevWork<R> &w = work<R>(s);
-    ck(cudaMemsetAsync(s->wf.sync, 0, kWfSyncWords * sizeof(unsigned), s->stream), "memset");
-    WfArgs<R> a{};
-    a.g = s->g;
-    a.buf[0] = st[0].rec;
-    a.buf[1] = st[1].rec;
-    a.wk = w;
-    a.gbuf[0] = w.grec;
-    a.gbuf[1] = s->wf.grec2;
-    a.sc = s->wf;
-    a.gas = s->gas;
-    a.cfl = s->sc.cfl;
-    for (int k = 0; k < 16; ++k) a.alpha[k] = s->sc.rk[k];
-    a.nst = s->sc.rk_level;
-    a.nopi = a.nst + (s->sc.order == 2 ? 1 : 0);
-    a.nops = (int64_t)n_iter * a.nopi;
-    a.n_iter = n_iter;
-    a.flux = s->sc.flux;
-    a.grad = s->sc.grad;
-    a.celllim = s->celllim;
-    a.in_buf = s->cur;
-    a.wait_ns = s->wait_ns;
-    ck(Ops<R>::wavefront(s->dim, s->rec, s->sc.limiter, a, s->wf_blocks, s->stream), "wavefront launch");
-    s->cur = (int)((s->cur + (int64_t)n_iter * a.nst) & 1);
+    const size_t row = (size_t)s->sc.rk_level * s->res.nitems * 2 * s->nv * sizeof(double);
+    const int most = (int)std::min<size_t>(std::max<size_t>(kResRowsMax / row, 1), 1 << 24);
+    const size_t need = row * (size_t)std::min(n_iter, most);
+    if (need > s->res_rows_cap) {
+        ck(cudaStreamSynchronize(s->stream), "stream sync");
+        s->dfree(s->res.rows);
+        s->res.rows = nullptr;
+        s->res_rows_cap = 0;
+        s->res.rows = (double *)s->dalloc_bytes(need);
+        s->res_rows_cap = need;
+    }
+    for (int done = 0; done < n_iter;) {
+        const int n = std::min(n_iter - done, most);
+        const uint32_t stages = (uint32_t)n * (uint32_t)s->sc.rk_level;
+        if (s->res_dirty || s->res_tag > 0x7fffffffu - stages || s->res_ptag > 0x7fffffffu - (uint32_t)n) {
+            for (auto p : s->res_state) ck(cudaMemsetAsync(p, 0, s->res_state_bytes, s->stream), "memset");
+            if (s->res_proj) ck(cudaMemsetAsync(s->res_proj, 0, s->res_proj_bytes, s->stream), "memset");
+            ck(cudaMemsetAsync(s->res.sync, 0, kWfSyncWords * sizeof(unsigned), s->stream), "memset");
+            s->res_tag = s->res_ptag = s->res_arrived = 0;
+            s->res_dirty = false;
+        }
+        ResArgs<R> a{};
+        a.g = s->g;
+        a.in = st[s->cur].rec;
+        a.out = st[s->cur ^ 1].rec;
+        for (int b = 0; b < 2; ++b) a.state[b] = (uint64_t *)s->res_state[b];
+        a.proj = (uint64_t *)s->res_proj;
+        a.tag0 = s->res_tag;
+        a.ptag0 = s->res_ptag;
+        a.wk = work<R>(s);
+        a.wk.linf += (size_t)done * s->nv;
+        a.wk.l2 += (size_t)done * s->nv;
+        a.sc = s->res;
+        a.sc.arrive_target = s->res_arrived + (unsigned)s->res_blocks;
+        a.gas = s->gas;
+        a.cfl = s->sc.cfl;
+        a.dt_uniform = s->dt_uniform;
+        a.rcv = 1.0 / s->gas.cv;
+        for (int k = 0; k < 16; ++k) a.alpha[k] = s->sc.rk[k];
+        a.nst = s->sc.rk_level;
+        a.nopi = a.nst + (s->sc.order == 2 ? 1 : 0);
+        a.n_iter = n;
+        a.nops = n * a.nopi;
+        a.nops_stage = (int32_t)stages;
+        a.flux = s->sc.flux;
+        a.grad = s->sc.grad;
+        a.celllim = s->celllim;
+        a.lc = s->sc.lc;
+        a.wait_ns = s->wait_ns;
+        ck(Ops<R>::resident(s->dim, s->rec, s->sc.limiter, a, s->res_blocks, s->res_smem, s->stream),
+           "resident launch");
+        s->res_tag += stages + 1u;
+        s->res_ptag += (uint32_t)n + 1u;
+        s->res_arrived += (unsigned)s->res_blocks;
+        s->cur ^= 1;
+        done += n;
+        mark(K_CELL);
+    }
 }
 
 template <typename R, typename Mark>
 void iterations(psst_solver *s, int n_iter, Mark &&mark) {
     DevWork<R> &w = work<R>(s);
-    if (wavefront_active(s)) {
-        wavefront_run<R>(s, n_iter);
-        mark(K_CELL);
+    if (s->seq && resident_active(s)) {
+        resident_run<R>(s, n_iter, mark);
         return;
     }
     for (int it = 0; it < n_iter; ++it) {
@@ -780,7 +917,9 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
     reserve_norms<R>(s, n_iter);
     int64_t launches = 0;
     ck(cudaEventRecord(s->ev0, s->stream), "event");
-    if (s->use_graphs && !wavefront_active(s)) {  // a wavefront call is one launch already
+    if (resident_active(s)) {  // one launch, which writes every residual column
+        resident_run<R>(s, n_iter, [&](int) { ++launches; });
+    } else if (s->use_graphs) {
         const std::pair<int, int> key(n_iter, s->cur);
         auto it = s->graphs.find(key);
         if (it == s->graphs.end()) {
@@ -853,7 +992,7 @@ template <typename R>
 int64_t run_to_stop(psst_solver *s, int64_t max_iter, int chunk, double *res_linf, double *res_l2) {
     DevWork<R> &w = work<R>(s);
     if (!s->stop_on) raise(PSST_ERR_STATE, "psst_solver_run_to_stop: no stop rule set (psst_solver_set_stop_rule)");
-    if (wavefront_active(s)) raise(PSST_ERR_UNSUPPORTED, "psst_solver_run_to_stop: not with the sequential mode");
+    if (s->seq) raise(PSST_ERR_UNSUPPORTED, "psst_solver_run_to_stop: not with the sequential mode");
     if ((int64_t)chunk * s->sc.rk_level % 2)
         raise(PSST_ERR_ARG, "psst_solver_run_to_stop: chunk * RK stages must be even");
     reserve_norms<R>(s, chunk);
@@ -1342,27 +1481,12 @@ extern "C" psst_status psst_solver_create(const psst_grid *G, const psst_scheme 
         alloc_state<float>(s.get(), *G);
     else
         alloc_state<double>(s.get(), *G);
-    if (s->seq && sc->precision == 64 && L.cell_case.empty() && !L.wf_item_level.empty()) {
-        const int maxb = Ops<double>::wavefront_max_blocks(s->dim, s->rec, sc->limiter);
-        // CTA 0 folds the norms; the others take the work items of a step
-        s->wf_blocks = std::min(L.wf_max_class_items + 1, maxb);
-        if (s->wf_blocks >= 2) {  // the items need a CTA besides CTA 0
-            WfSched &w = s->wf;
-            w.period = L.wf_period;
-            w.nlevels = L.nlevels;
-            w.nitems = (int32_t)L.wf_item_level.size();
-            w.cells32 = s->upload(L.wf_cells32);
-            w.lowmask = s->upload(L.wf_lowmask);
-            w.item_level = s->upload(L.wf_item_level);
-            w.lvl_items = s->upload(L.wf_lvl_items);
-            w.ipart = s->dalloc<double>((size_t)2 * w.nitems * 2 * s->nv);
-            w.nacc = L.nlevels / L.wf_period + 3;
-            w.acc = s->dalloc<double>((size_t)w.nacc * 2 * s->nv);
-            w.grec2 = s->dalloc_bytes(Ops<double>::grad_rec_bytes(s->dim) * std::max(L.nint, 1));
-            ck(cudaMemset(w.grec2, 0, Ops<double>::grad_rec_bytes(s->dim) * std::max(L.nint, 1)), "memset");
-            w.sync = s->dalloc<unsigned>(kWfSyncWords);
-            s->wf_ready = true;
-        }
+    // the sequential mode at FP32 keeps the level walk
+    if (L.cell_case.empty() && !(s->seq && sc->precision == 32)) {
+        if (sc->precision == 32)
+            build_resident<float>(s.get());
+        else
+            build_resident<double>(s.get());
     }
     ck(cudaDeviceSynchronize(), "setup");
     *out = s.release();
@@ -1647,7 +1771,7 @@ extern "C" psst_status psst_solver_case_residuals(psst_solver *s, int n_iter, do
 extern "C" psst_status psst_solver_use_wavefront(psst_solver *s, int on) {
     PSST_API_BEGIN
     if (!s) raise(PSST_ERR_ARG, "null solver");
-    s->wf_on = on != 0;
+    s->res_on = on != 0;
     PSST_API_END
 }
 
@@ -1661,11 +1785,13 @@ extern "C" psst_status psst_solver_set_wait_limit(psst_solver *s, int64_t ns) {
 extern "C" psst_status psst_solver_schedule_info(const psst_solver *s, int64_t *info) {
     PSST_API_BEGIN
     if (!s || !info) raise(PSST_ERR_ARG, "psst_solver_schedule_info: null argument");
-    info[0] = wavefront_active(s) ? 1 : 0;
-    info[1] = s->L.wf_period;
-    info[2] = s->L.nlevels;
-    info[3] = (int64_t)s->L.wf_item_level.size();
-    info[4] = s->wf_blocks;
+    info[0] = resident_active(s) ? 1 : 0;
+    info[1] = s->L.res_period;
+    int32_t nlevels = s->L.nlevels;
+    if (!s->seq) cell_levels(s->L, nlevels);  // the parallel modes do not keep them
+    info[2] = nlevels;
+    info[3] = (int64_t)s->L.res_item_level.size();
+    info[4] = s->res_blocks;
     PSST_API_END
 }
 
