@@ -71,11 +71,13 @@ struct Ops {
     static void loop_control(int dim, const DevGrid &g, const DevWork<R> &wk, const CaseStop &cs, LoopCtl *ctl,
                              int chunk, cudaGraphConditionalHandle h, cudaStream_t s);
     // A whole call as one cooperative launch of nblocks CTAs (k_resident).
-    static cudaError_t resident(int dim, int rec, int lim, const ResArgs<R> &a, int nblocks, size_t smem,
+    static cudaError_t resident(int dim, int rec, int lim, const ResArgs<R> &a, int nblocks, bool more, size_t smem,
                                 cudaStream_t s);
-    // co-resident CTAs of that kernel on the current device, with up to `want`
-    // items of a CTA in shared memory (*items of them, *smem bytes)
-    static int resident_max_blocks(int dim, int rec, int lim, int rounds, int want, int *items, size_t *smem);
+    // co-resident CTAs of that kernel (more: the build with more CTAs an SM) on the
+    // current device, with up to `want` items of a CTA in shared memory (*items of
+    // them, *smem bytes)
+    static int resident_max_blocks(int dim, int rec, int lim, int rounds, bool more, int want, int *items,
+                                   size_t *smem);
     static size_t resident_store_bytes(int dim, int rec, int rounds);  // ItemStore of one item
     // sizes of its tables and buffers for nint cells in nitems items
     struct ResidentBytes {

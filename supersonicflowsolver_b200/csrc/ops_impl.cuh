@@ -281,31 +281,33 @@ void Ops<R>::loop_control(int dim, const DevGrid &g, const DevWork<R> &wk, const
 
 // ---- a whole call as one persistent launch ----
 template <typename R, int DIM>
-static cudaError_t resident_d(int rec, int lim, const ResArgs<R> &a, int nb, size_t smem, cudaStream_t s) {
-    if (rec == 0) return res_launch<R, DIM, 0, 1>(a, nb, smem, s);
-    if (rec == 2) return res_launch<R, DIM, 2, 1>(a, nb, smem, s);
-    if (lim == 1) return res_launch<R, DIM, 1, 1>(a, nb, smem, s);
-    if (lim == 2) return res_launch<R, DIM, 1, 2>(a, nb, smem, s);
-    return res_launch<R, DIM, 1, 3>(a, nb, smem, s);
+static cudaError_t resident_d(int rec, int lim, const ResArgs<R> &a, int nb, bool more, size_t smem, cudaStream_t s) {
+    if (rec == 0) return res_launch<R, DIM, 0, 1>(a, nb, more, smem, s);
+    if (rec == 2) return res_launch<R, DIM, 2, 1>(a, nb, more, smem, s);
+    if (lim == 1) return res_launch<R, DIM, 1, 1>(a, nb, more, smem, s);
+    if (lim == 2) return res_launch<R, DIM, 1, 2>(a, nb, more, smem, s);
+    return res_launch<R, DIM, 1, 3>(a, nb, more, smem, s);
 }
 template <typename R, int DIM>
-static int resident_max_d(int rec, int lim, int rounds, int want, int *items, size_t *smem) {
-    if (rec == 0) return res_max_blocks<R, DIM, 0, 1>(rounds, want, items, smem);
-    if (rec == 2) return res_max_blocks<R, DIM, 2, 1>(rounds, want, items, smem);
-    if (lim == 1) return res_max_blocks<R, DIM, 1, 1>(rounds, want, items, smem);
-    if (lim == 2) return res_max_blocks<R, DIM, 1, 2>(rounds, want, items, smem);
-    return res_max_blocks<R, DIM, 1, 3>(rounds, want, items, smem);
+static int resident_max_d(int rec, int lim, int rounds, bool more, int want, int *items, size_t *smem) {
+    if (rec == 0) return res_max_blocks<R, DIM, 0, 1>(rounds, more, want, items, smem);
+    if (rec == 2) return res_max_blocks<R, DIM, 2, 1>(rounds, more, want, items, smem);
+    if (lim == 1) return res_max_blocks<R, DIM, 1, 1>(rounds, more, want, items, smem);
+    if (lim == 2) return res_max_blocks<R, DIM, 1, 2>(rounds, more, want, items, smem);
+    return res_max_blocks<R, DIM, 1, 3>(rounds, more, want, items, smem);
 }
 
 template <typename R>
-cudaError_t Ops<R>::resident(int dim, int rec, int lim, const ResArgs<R> &a, int nb, size_t smem, cudaStream_t s) {
-    return dim == 2 ? resident_d<R, 2>(rec, lim, a, nb, smem, s) : resident_d<R, 3>(rec, lim, a, nb, smem, s);
+cudaError_t Ops<R>::resident(int dim, int rec, int lim, const ResArgs<R> &a, int nb, bool more, size_t smem,
+                             cudaStream_t s) {
+    return dim == 2 ? resident_d<R, 2>(rec, lim, a, nb, more, smem, s) : resident_d<R, 3>(rec, lim, a, nb, more, smem, s);
 }
 
 template <typename R>
-int Ops<R>::resident_max_blocks(int dim, int rec, int lim, int rounds, int want, int *items, size_t *smem) {
-    return dim == 2 ? resident_max_d<R, 2>(rec, lim, rounds, want, items, smem)
-                    : resident_max_d<R, 3>(rec, lim, rounds, want, items, smem);
+int Ops<R>::resident_max_blocks(int dim, int rec, int lim, int rounds, bool more, int want, int *items,
+                                size_t *smem) {
+    return dim == 2 ? resident_max_d<R, 2>(rec, lim, rounds, more, want, items, smem)
+                    : resident_max_d<R, 3>(rec, lim, rounds, more, want, items, smem);
 }
 
 template <typename R>

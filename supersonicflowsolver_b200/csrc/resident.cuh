@@ -18,9 +18,9 @@
 // that the reference updates first); all of these come earlier in that order,
 // and all CTAs are co-resident, so the oldest unfinished pair can always run.
 //
-// What a neighbour needs is published in words of one value and one tag, each
-// written and read whole by one 16-byte (FP64) or 8-byte (FP32) relaxed access:
-// the reader polls the word itself until the tag says it holds the operation
+// What a neighbour needs is published in records whose every 64-bit word holds
+// its own tag (Record below): the reader polls the record itself until the tags
+// say that it holds the operation
 // asked for. So a result costs one store and one load through L2 (541 cycles
 // one way, measured between two SMs) -- no fence, no flag, no barrier. States
 // are double-buffered by stage parity and gradient projections single-buffered:
@@ -40,6 +40,14 @@
 // lane. One lane a cell, four faces interleaved, was measured too: 3640
 // instructions an operation and twice the time.
 //
+// Measured (a whole call, set_state to norms, launch-by-launch or one-CTA-a-level
+// chain before -> now): 60 x 20 FP64, one iteration 155 -> 111 us; 120 x 40 FP64,
+// 100 iterations 5.25 -> 1.99 ms; 240 x 80 FP32, 50 iterations 2.11 -> 1.49 ms;
+// sequential 240 x 80 (first order, 300) 8.55 -> 4.16 ms and 120 x 40 (30) 4.15 -> 1.52 ms. An operation
+// of the 120 x 40 case takes some 8300 cycles: 900 for the static data, 900
+// waiting for neighbours, 2400 fluxes, 800 the sums over the faces, 1450 update and
+// publication, 550 ghosts, 350 norms, 900 the loop and its barrier.
+//
 // Every wait is bounded: one longer than wait_ns sets the abort flag and
 // ERR_TIMEOUT, and every warp leaves at its next wait.
 #pragma once
@@ -48,17 +56,6 @@
 #include "exact.cuh"
 #include "kernels.cuh"
 #include "ops.hpp"
-
-// CTAs per SM the kernel is built for (register cap 65536 / (128 x this)).
-#ifndef PSST_RES_MINB_F64
-#define PSST_RES_MINB_F64 2
-#endif
-#ifndef PSST_RES_MINB_F64_3D
-#define PSST_RES_MINB_F64_3D 2
-#endif
-#ifndef PSST_RES_MINB_F32
-#define PSST_RES_MINB_F32 5
-#endif
 
 namespace psst {
 
@@ -1221,13 +1218,16 @@ __device__ __forceinline__ void res_columns(const ResArgs<R> &a) {
     }
 }
 
-template <typename R, int DIM>
+// Two builds of the kernel: few CTAs an SM with the registers the code wants, and
+// one more an SM with some spilled, for meshes that need that many CTAs to have
+// one item each (a second item doubles an operation).
+template <typename R, int DIM, bool MORE>
 constexpr int res_min_blocks() {
-    return sizeof(R) == 4 ? PSST_RES_MINB_F32 : DIM == 2 ? PSST_RES_MINB_F64 : PSST_RES_MINB_F64_3D;
+    return sizeof(R) == 4 ? (MORE ? 5 : 4) : DIM == 2 && MORE ? 3 : 2;
 }
 
-template <typename R, int DIM, int REC, int LIM>
-__global__ void __launch_bounds__(kWfBlock, res_min_blocks<R, DIM>()) k_resident(const __grid_constant__ ResArgs<R> a) {
+template <typename R, int DIM, int REC, int LIM, bool MORE>
+__global__ void __launch_bounds__(kWfBlock, res_min_blocks<R, DIM, MORE>()) k_resident(const __grid_constant__ ResArgs<R> a) {
     constexpr int NV = DIM + 2;
     extern __shared__ __align__(16) char res_smem[];
     __shared__ NormRows<NV> rows;
@@ -1289,18 +1289,19 @@ __global__ void __launch_bounds__(kWfBlock, res_min_blocks<R, DIM>()) k_resident
 }
 
 template <typename R, int DIM, int REC, int LIM>
-cudaError_t res_launch(const ResArgs<R> &a, int nblocks, size_t smem, cudaStream_t s) {
+cudaError_t res_launch(const ResArgs<R> &a, int nblocks, bool more, size_t smem, cudaStream_t s) {
     void *args[] = {const_cast<ResArgs<R> *>(&a)};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&k_resident<R, DIM, REC, LIM>), dim3(nblocks),
-                                       dim3(kWfBlock), args, smem, s);
+    const void *kern = more ? reinterpret_cast<const void *>(&k_resident<R, DIM, REC, LIM, true>)
+                            : reinterpret_cast<const void *>(&k_resident<R, DIM, REC, LIM, false>);
+    return cudaLaunchCooperativeKernel(kern, dim3(nblocks), dim3(kWfBlock), args, smem, s);
 }
 
 // Most co-resident CTAs with the most items kept in shared memory (at most
 // want): keeping the item on chip comes after having another CTA.
 template <typename R, int DIM, int REC, int LIM>
-int res_max_blocks(int rounds, int want, int *items, size_t *smem) {
+int res_max_blocks(int rounds, bool more, int want, int *items, size_t *smem) {
     int dev = 0, nsm = 0, lim = 0;
-    auto kern = k_resident<R, DIM, REC, LIM>;
+    auto kern = more ? k_resident<R, DIM, REC, LIM, true> : k_resident<R, DIM, REC, LIM, false>;
     cudaFuncAttributes at{};
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;

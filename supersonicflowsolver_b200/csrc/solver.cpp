@@ -87,10 +87,9 @@ struct Layout {
 std::vector<int32_t> cell_levels(const Layout &L, int32_t &nlevels);
 void build_resident_items(Layout &L, const std::vector<int32_t> &level, bool seq);
 
-// Most cells for which the parallel modes run as one resident launch: beyond
-// it every CTA has several items to work through per operation, and the pass
-// kernels, which form each interior face's flux once, are faster.
-constexpr int32_t kResidentMaxCells = 40000;
+// Cells beyond which the parallel modes never run as one resident launch
+// (build_resident decides below it).
+constexpr int32_t kResidentMaxCells = 1 << 16;
 
 void build_layout(const psst_grid &G, const psst_scheme &sc, Layout &L) {
     const int dim = G.dim;
@@ -535,6 +534,7 @@ struct psst_solver {
     bool res_ready = false, res_on = true, res_dirty = false;
     ResSched res{};
     int res_blocks = 0;
+    bool res_more = false;  // the build with more CTAs an SM
     size_t res_smem = 0;
     void *res_state[2] = {nullptr, nullptr}, *res_proj = nullptr;
     size_t res_state_bytes = 0, res_proj_bytes = 0, res_rows_cap = 0;
@@ -753,8 +753,9 @@ void one_stage(psst_solver *s, int k, int it_slot, bool gather, Mark &&mark) {
 bool resident_active(const psst_solver *s) { return s->res_ready && s->res_on; }
 
 // Bytes of norm rows that one resident launch may write; a longer call is cut
-// into several launches.
-constexpr size_t kResRowsMax = (size_t)256 << 20;
+// into several launches (each some 10 us, for at least 50 iterations of the
+// largest mesh taken; 256 MB put 1 ms of allocation into a solver's first call).
+constexpr size_t kResRowsMax = (size_t)16 << 20;
 
 // Tables and buffers of the resident launch, if the kernel fits the device.
 template <typename R>
@@ -766,8 +767,24 @@ void build_resident(psst_solver *s) {
     int maxk = 1;
     for (int32_t d = 0; d < L.nint; ++d) maxk = std::max(maxk, L.csr_ptr[d + 1] - L.csr_ptr[d]);
     w.rounds = (maxk + 3) / 4;
-    int items = 0;
-    const int maxb = Ops<R>::resident_max_blocks(s->dim, s->rec, s->sc.limiter, w.rounds, 2, &items, &s->res_smem);
+    int items = 0, maxb = 0;
+    for (const bool more : {false, true}) {  // the build whose CTAs suffice for an item each
+        if (more && maxb >= nitems) break;
+        s->res_more = more;
+        maxb = Ops<R>::resident_max_blocks(s->dim, s->rec, s->sc.limiter, w.rounds, more, 2, &items, &s->res_smem);
+    }
+    // The parallel modes: up to the sizes where it is the faster form. Every
+    // interior face's flux is formed twice and a cell's faces take turns four at a
+    // time, against ten launches an iteration: us an iteration, resident / passes,
+    // HLLC MUSCL RK4: FP64 quads 4800 24.4 / 52.2, 10800 44.1 / 57.2, 19200 (two
+    // items a CTA) 72 / 65; FP32 quads 4800 17.9 / 38.9, 19200 33.4 / 44.5, 30000
+    // 58 / 46; with more than four faces a cell: FP64 hanging nodes 4906 55 / 64,
+    // 11298 126 / 67, hexes 2304 64.5 / 63.5; FP32 hexes 18432 46.8 / 57.8.
+    if (!s->seq) {
+        const bool f32 = sizeof(R) == 4, many = w.rounds > 1;
+        if (f32 ? many && s->res_more : many && (s->dim == 3 || nitems > maxb / 2)) return;
+        if (nitems > maxb) return;
+    }
     if (maxb <= 0) return;
     s->res_blocks = std::min(nitems, maxb);
     w.period = L.res_period;
@@ -791,43 +808,68 @@ void build_resident(psst_solver *s) {
         most = std::max(most, (int)own.size() - ptr.back());
         ptr.push_back((int32_t)own.size());
     }
-    w.own_ptr = s->upload(ptr);
-    w.own = s->upload(own);
-    w.cells32 = s->upload(L.res_cells32);
-    if (most > items)
-        w.store = (char *)s->dalloc_bytes(nitems * Ops<R>::resident_store_bytes(s->dim, s->rec, w.rounds));
-    w.sync = s->dalloc<unsigned>(kWfSyncWords);
-    const auto bytes = Ops<R>::resident_bytes(s->dim, L.nint, nitems, w.rounds);
-    s->res_state_bytes = bytes.state;
-    for (auto &p : s->res_state) p = s->dalloc_bytes(bytes.state);
-    if (s->sc.order == 2) {
-        s->res_proj_bytes = bytes.proj;
-        s->res_proj = s->dalloc_bytes(bytes.proj);
-    }
-    // static lane data, from arrays that only its construction needs
+    // one block of device memory and one copy: the host tables (the last three are
+    // read by the construction of the static data only), then the buffers
     std::vector<int32_t> pos(L.nint);
     for (size_t i = 0; i < L.res_cells32.size(); ++i)
         if (L.res_cells32[i] >= 0) pos[L.res_cells32[i]] = (int32_t)i;
-    void *lanes = s->dalloc_bytes(bytes.lanes), *cells = s->dalloc_bytes((size_t)nitems * 32 * 2 * sizeof(double));
-    int32_t *d_mate = s->upload(mate_entries(L)), *d_pos = s->upload(pos);
-    uint32_t *d_low = L.res_lowmask.empty() ? nullptr : s->upload(L.res_lowmask);
-    Ops<R>::resident_build(s->dim, s->rec, s->sc.order == 2 ? s->sc.grad : 0, s->g, w.cells32, d_low, d_mate, d_pos,
-                           nitems, w.rounds, lanes, cells, s->stream);
+    const std::vector<int32_t> mate = mate_entries(L);
+    const auto bytes = Ops<R>::resident_bytes(s->dim, L.nint, nitems, w.rounds);
+    size_t off = 0;
+    auto take = [&](size_t n) {
+        const size_t at = off;
+        off += (n + 255) / 256 * 256;
+        return at;
+    };
+    const size_t o_ptr = take(ptr.size() * 4), o_own = take(own.size() * sizeof(int2)),
+                 o_cells = take(L.res_cells32.size() * 4), o_low = take(L.res_lowmask.size() * 4),
+                 o_mate = take(mate.size() * 4), o_pos = take(pos.size() * 4), tables = off;
+    const size_t o_sync = take(kWfSyncWords * sizeof(unsigned)), o_state0 = take(bytes.state), o_state1 = take(bytes.state),
+                 o_proj = take(s->sc.order == 2 ? bytes.proj : 0), o_faces = take(bytes.lanes),
+                 o_vol = take((size_t)nitems * 32 * 2 * sizeof(double)),
+                 o_store = take(most > items ? nitems * Ops<R>::resident_store_bytes(s->dim, s->rec, w.rounds) : 0);
+    char *base = (char *)s->dalloc_bytes(off);
+    std::vector<char> host(tables);
+    auto put = [&](size_t at, const void *p, size_t n) {
+        if (n) std::memcpy(host.data() + at, p, n);
+    };
+    put(o_ptr, ptr.data(), ptr.size() * 4);
+    put(o_own, own.data(), own.size() * sizeof(int2));
+    put(o_cells, L.res_cells32.data(), L.res_cells32.size() * 4);
+    put(o_low, L.res_lowmask.data(), L.res_lowmask.size() * 4);
+    put(o_mate, mate.data(), mate.size() * 4);
+    put(o_pos, pos.data(), pos.size() * 4);
+    ck(cudaMemcpyAsync(base, host.data(), tables, cudaMemcpyHostToDevice, s->stream), "resident tables");
+    w.own_ptr = (const int32_t *)(base + o_ptr);
+    w.own = (const int2 *)(base + o_own);
+    w.cells32 = (const int32_t *)(base + o_cells);
+    w.sync = (unsigned *)(base + o_sync);
+    w.faces = (const uint4 *)(base + o_faces);
+    w.cells = (const double2 *)(base + o_vol);
+    w.store = base + o_store;
+    s->res_state_bytes = bytes.state;
+    s->res_state[0] = base + o_state0;
+    s->res_state[1] = base + o_state1;
+    if (s->sc.order == 2) {
+        s->res_proj_bytes = bytes.proj;
+        s->res_proj = base + o_proj;
+    }
+    Ops<R>::resident_build(s->dim, s->rec, s->sc.order == 2 ? s->sc.grad : 0, s->g, w.cells32,
+                           L.res_lowmask.empty() ? nullptr : (const uint32_t *)(base + o_low),
+                           (const int32_t *)(base + o_mate), (const int32_t *)(base + o_pos), nitems, w.rounds,
+                           base + o_faces, base + o_vol, s->stream);
     ck(cudaGetLastError(), "resident tables");
     ck(cudaStreamSynchronize(s->stream), "resident tables");
-    s->dfree(d_mate);
-    s->dfree(d_pos);
-    s->dfree(d_low);
-    w.faces = (const uint4 *)lanes;
-    w.cells = (const double2 *)cells;
     s->res_dirty = true;  // tags cleared before the first launch
     s->res_ready = true;
 }
 
 // n_iter iterations as cooperative launches of the resident kernel (one,
-// unless the norm rows of the call exceed kResRowsMax).
+// unless the norm rows of the call exceed kResRowsMax). False, with nothing
+// done, where the device does not take a launch of that size (a share of the
+// device smaller than it reports) and the passes can run the call instead.
 template <typename R, typename Mark>
-void resident_run(psst_solver *s, int n_iter, Mark &&mark) {
+bool resident_run(psst_solver *s, int n_iter, Mark &&mark) {
     DevState<R> *st = states<R>(s);
     const size_t row = (size_t)s->sc.rk_level * s->res.nitems * 2 * s->nv * sizeof(double);
     const int most = (int)std::min<size_t>(std::max<size_t>(kResRowsMax / row, 1), 1 << 24);
@@ -878,8 +920,14 @@ void resident_run(psst_solver *s, int n_iter, Mark &&mark) {
         a.celllim = s->celllim;
         a.lc = s->sc.lc;
         a.wait_ns = s->wait_ns;
-        ck(Ops<R>::resident(s->dim, s->rec, s->sc.limiter, a, s->res_blocks, s->res_smem, s->stream),
-           "resident launch");
+        const cudaError_t e =
+            Ops<R>::resident(s->dim, s->rec, s->sc.limiter, a, s->res_blocks, s->res_more, s->res_smem, s->stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge && !s->seq && done == 0) {
+            cudaGetLastError();
+            s->res_ready = false;
+            return false;
+        }
+        ck(e, "resident launch");
         s->res_tag += stages + 1u;
         s->res_ptag += (uint32_t)n + 1u;
         s->res_arrived += (unsigned)s->res_blocks;
@@ -887,6 +935,7 @@ void resident_run(psst_solver *s, int n_iter, Mark &&mark) {
         done += n;
         mark(K_CELL);
     }
+    return true;
 }
 
 template <typename R, typename Mark>
@@ -917,8 +966,9 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
     reserve_norms<R>(s, n_iter);
     int64_t launches = 0;
     ck(cudaEventRecord(s->ev0, s->stream), "event");
-    if (resident_active(s)) {  // one launch, which writes every residual column
-        resident_run<R>(s, n_iter, [&](int) { ++launches; });
+    const auto count = [&](int) { ++launches; };
+    if (resident_active(s) && resident_run<R>(s, n_iter, count)) {
+        // one launch, which wrote every residual column
     } else if (s->use_graphs) {
         const std::pair<int, int> key(n_iter, s->cur);
         auto it = s->graphs.find(key);
@@ -927,7 +977,7 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
             cudaGraph_t gr = nullptr;
             try {
                 zero_norms<R>(s, n_iter);
-                iterations<R>(s, n_iter, [&](int) { ++launches; });
+                iterations<R>(s, n_iter, count);
             } catch (...) {
                 cudaStreamEndCapture(s->stream, &gr);
                 if (gr) cudaGraphDestroy(gr);
@@ -947,7 +997,7 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
         ck(cudaGraphLaunch(it->second, s->stream), "graph launch");
     } else {
         zero_norms<R>(s, n_iter);
-        iterations<R>(s, n_iter, [&](int) { ++launches; });
+        iterations<R>(s, n_iter, count);
     }
     ck(cudaEventRecord(s->ev1, s->stream), "event");
     ck(cudaGetLastError(), "kernel launch");
@@ -1790,7 +1840,7 @@ extern "C" psst_status psst_solver_schedule_info(const psst_solver *s, int64_t *
     int32_t nlevels = s->L.nlevels;
     if (!s->seq) cell_levels(s->L, nlevels);  // the parallel modes do not keep them
     info[2] = nlevels;
-    info[3] = (int64_t)s->L.res_item_level.size();
+    info[3] = s->res_ready || s->seq ? (int64_t)s->L.res_item_level.size() : 0;
     info[4] = s->res_blocks;
     PSST_API_END
 }
