@@ -753,9 +753,8 @@ void one_stage(psst_solver *s, int k, int it_slot, bool gather, Mark &&mark) {
 bool resident_active(const psst_solver *s) { return s->res_ready && s->res_on; }
 
 // Bytes of norm rows that one resident launch may write; a longer call is cut
-// into several launches (each some 10 us, for at least 50 iterations of the
-// largest mesh taken; 256 MB put 1 ms of allocation into a solver's first call).
-constexpr size_t kResRowsMax = (size_t)16 << 20;
+// into several launches.
+constexpr size_t kResRowsMax = (size_t)256 << 20;
 
 // Tables and buffers of the resident launch, if the kernel fits the device.
 template <typename R>

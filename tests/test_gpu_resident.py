@@ -94,7 +94,7 @@ def test_resident_equals_passes(tmp_path, mesh, ckw, bits):
 
 
 def test_long_call_in_several_launches(tmp_path):
-    """120 x 80 quads: an iteration's norm rows are 77 kB, so 300 iterations take two launches."""
+    """120 x 80 quads: an iteration's norm rows are 77 kB, so 3600 iterations take two launches."""
     m = meshgen.wedge2d(120, 80, 12.0)
     path, d, name = make_case(tmp_path, m, max_iter=1, flux=2, order=1, lc=1, rk_level=4, mach=2.5)
     g = Grid.read_fluent(path)
@@ -103,9 +103,9 @@ def test_long_call_in_several_launches(tmp_path):
     a, b = Solver(g, sc), Solver(g, sc)
     a.set_state(prim)
     b.set_state(prim)
-    la, ra = a.explicit_solve(300)
+    la, ra = a.explicit_solve(3600)
     assert a.last_stats()[0] == 2
-    parts = [b.explicit_solve(100) for _ in range(3)]
+    parts = [b.explicit_solve(1200) for _ in range(3)]
     assert np.array_equal(la, np.concatenate([p[0] for p in parts]))
     assert np.array_equal(ra, np.concatenate([p[1] for p in parts]))
     assert np.array_equal(a.get_state(), b.get_state())
