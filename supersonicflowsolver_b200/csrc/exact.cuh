@@ -26,7 +26,7 @@
 // plain operators otherwise.
 //
 // FP32: the approximate reciprocal (square root) with one residual correction,
-// within 0.51 ulp of the exact value.
+// within 0.51 ulp of the exact value. rn_div is the rounded quotient, as above.
 #pragma once
 #include <cstdint>
 
@@ -85,6 +85,14 @@ __device__ __forceinline__ float lin_quot(float a, float b, float y) {
 template <typename R>
 __device__ __forceinline__ R lin_div(R a, R b) {
     return lin_quot(a, b, lin_recip(b));
+}
+// the same with the reciprocal corrected first, which rounds it correctly:
+// the bits of a / b for 2^-126 <= 1 / b and 2^-100 <= |a|, |a / b| (smaller
+// quantities lose bits of the residual), and for a = 0 up to the sign of a -0
+__device__ __forceinline__ float rn_div(float a, float b) {
+    float y = lin_recip(b);
+    y = fmaf(fmaf(-b, y, 1.0f), y, y);
+    return lin_quot(a, b, y);
 }
 __device__ __forceinline__ double lin_sqrt(double x) {
     double y;

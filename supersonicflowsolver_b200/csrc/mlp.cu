@@ -8,9 +8,9 @@
 //        4 * 30 + 4 = 124 values, zero-padded to 128
 //   h1 = silu(W1 f + b1), h_l = silu(W_l h_{l-1} + b_l) for l = 2..5
 //   y  = W6 h5 + b6                                  (4 outputs: rho, u, v, p)
-// Loss: mean over points and outputs of (y - target)^2.
+// Loss: mean over points and outputs of (y - target)^2. Its kernels: mlp_net.cuh.
 //
-// GEMM kernels: one CTA computes a 128 x NT tile of D = A . B^T, A [M x K],
+// GEMM kernels (psst_tc_gemm_bf16): one CTA computes a 128 x NT tile of D = A . B^T, A [M x K],
 // B [N x K] given by element strides (so transposed operands need no copy).
 // K is walked in 64-wide chunks, four tcgen05.mma.kind::f16 (M = 128, N = NT,
 // K = 16) per chunk, issued by one thread, FP32 accumulators in tensor memory.
@@ -28,12 +28,12 @@
 //    core matrices), two stages, transposing operands contiguous along M/N in
 //    registers, 8 x 8 at a time.
 // The epilogue reads the accumulator with tcgen05.ld (one row per thread, 32
-// columns at a time), applies bias / SiLU / SiLU-derivative and writes each
-// row segment with 16-byte stores. Split-K over gridDim.z writes FP32
-// partials that a second kernel sums in a fixed order (deterministic). Every
-// mbarrier wait is bounded; a wait that runs out drains the MMAs and copies in
-// flight before the CTA frees its tensor memory and reports the timeout.
+// columns at a time) and writes each row segment with 16-byte stores. Split-K over
+// gridDim.z writes FP32 partial sums. Every mbarrier wait is bounded; a wait that
+// runs out drains the MMAs and copies in flight before the CTA frees its tensor
+// memory and reports the timeout.
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <memory>
@@ -44,6 +44,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime_api.h>
 
+#include "exact.cuh"
 #include "host.hpp"
 
 namespace {
@@ -56,7 +57,6 @@ constexpr int kThreads = 128;
 constexpr unsigned kWaitLimit = 1u << 26;  // mbarrier polls before giving up (~seconds)
 constexpr int kStages = 2;                 // operand stages in shared memory
 
-enum Epi { EPI_NONE = 0, EPI_SILU = 1, EPI_DSILU = 2 };
 enum MlpErr { MLP_ERR_TIMEOUT = 1 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -153,10 +153,21 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float dsilu(float z) {
-    const float s = 1.0f / (1.0f + expf(-z));
-    return s * (1.0f + z * (1.0f - s));
+// 16 columns, which are there after tmem_wait(r).
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t r[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_wait(uint32_t r[16]) {  // r: no use of the registers moves ahead of the wait
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
 }
 
 struct GemmArgs {
@@ -165,16 +176,11 @@ struct GemmArgs {
     const bf16 *B;
     int64_t b_sn, b_sk;  // B[n][k] = B[n * b_sn + k * b_sk]
     int M, N, K, k_split;
-    const float *bias;   // [N] or null
-    int epi;             // Epi
-    const bf16 *Zin;     // EPI_DSILU: pre-activation [M][N] (row stride d_sm)
-    float *D32;          // FP32 output [splits][M][d_sm] (or null)
-    bf16 *D16;           // BF16 output [M][d_sm] (or null)
-    bf16 *Z16;           // BF16 pre-activation output [M][d_sm] (EPI_SILU, or null)
+    float *D32;  // FP32 output [splits][M][d_sm]
     int64_t d_sm;
     int *err;
     unsigned wait_polls;  // bound of the first wait that runs out (kWaitLimit; 0 gives up at once)
-    int vec;              // outputs and Zin 16-byte aligned, d_sm % 8 == 0: 16-byte epilogue stores
+    int vec;              // output 16-byte aligned, d_sm % 4 == 0: 16-byte epilogue stores
 };
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -182,45 +188,28 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-constexpr int kEpiWarpBytes = 8192;  // per warp: a 32 x 32 FP32 tile (4 KB) + two BF16 tiles (2 KB each)
+constexpr int kEpiWarpBytes = 4096;  // per warp: a 32 x 32 FP32 tile
 
-// Swizzled 32-row tiles in shared memory: 16-byte chunk c of row r of an FP32
-// tile (128-byte rows) at r * 128 + (c ^ (r & 7)) * 16, of a BF16 tile
-// (64-byte rows) at r * 64 + (c ^ ((r >> 1) & 3)) * 16. A warp writing one
-// row per lane, or reading 512 contiguous bytes, hits every bank 4 times.
+// Swizzled 32-row FP32 tile in shared memory: 16-byte chunk c of row r at
+// r * 128 + (c ^ (r & 7)) * 16. A warp writing one row per lane, or reading 512
+// contiguous bytes, hits every bank 4 times.
 __device__ __forceinline__ uint4 *tile32(unsigned char *t, int r, int c) {
     return reinterpret_cast<uint4 *>(t + r * 128 + ((c ^ (r & 7)) << 4));
 }
-__device__ __forceinline__ uint4 *tile16(unsigned char *t, int r, int c) {
-    return reinterpret_cast<uint4 *>(t + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
-}
-
-// Writes the warp's BF16 tile (rows m0w.., columns nb..nb+31) to g (row
-// stride ld): each store instruction covers 8 rows x 64 bytes.
-__device__ __forceinline__ void tile16_store(unsigned char *t, bf16 *g, int64_t ld, int m0w, int M, int nb) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = 8 * i + (lane >> 2), c = lane & 3;
-        if (m0w + r < M) *reinterpret_cast<uint4 *>(g + (int64_t)(m0w + r) * ld + nb + 8 * c) = *tile16(t, r, c);
-    }
-    __syncwarp();
-}
 
 // Epilogue: thread t holds accumulator row m0 + t (TMEM lane t) and handles it
-// 32 columns at a time: bias and activation in registers; then, with a.vec and
-// the whole segment inside N, each warp passes its 32 x 32 block through its
-// shared-memory tiles so that global loads and stores cover whole rows (16
-// bytes per lane); otherwise element by element. `tiles`: kEpiWarpBytes per
-// warp of free shared memory.
+// 32 columns at a time; with a.vec and the whole segment inside N, each warp
+// passes its 32 x 32 block through its shared-memory tile so that global stores
+// cover whole rows (16 bytes per lane); otherwise element by element. `tiles`:
+// kEpiWarpBytes per warp of free shared memory.
 template <int NT>
 __device__ __forceinline__ void epilogue(const GemmArgs &a, uint32_t tmem, int m0, int n0, bool empty,
                                          unsigned char *tiles) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int m0w = m0 + 32 * warp, m = m0w + lane;
     const uint32_t lanes = (uint32_t)(32 * warp) << 16;  // this warp's 32 TMEM lanes
-    unsigned char *tf = tiles + warp * kEpiWarpBytes, *th = tf + 4096, *tz = th + 2048;
+    unsigned char *tf = tiles + warp * kEpiWarpBytes;
+    float *out = a.D32 + (int64_t)blockIdx.z * a.M * a.d_sm;
     for (int c0 = 0; c0 < NT && n0 + c0 < a.N; c0 += 32) {
         float v[32];
         if (!empty)
@@ -229,82 +218,24 @@ __device__ __forceinline__ void epilogue(const GemmArgs &a, uint32_t tmem, int m
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0.0f;
         const int nb = n0 + c0, nn = min(32, a.N - nb);
-        if (a.bias)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-                if (i < nn) v[i] += a.bias[nb + i];
         if (a.vec && nn == 32) {  // warp-uniform
-            if (a.D32) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    *tile32(tf, lane, j) = make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]),
-                                                      __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3]));
-                __syncwarp();
-                float *d32 = a.D32 + (int64_t)blockIdx.z * a.M * a.d_sm;
+            for (int j = 0; j < 8; ++j)
+                *tile32(tf, lane, j) = make_uint4(__float_as_uint(v[4 * j]), __float_as_uint(v[4 * j + 1]),
+                                                  __float_as_uint(v[4 * j + 2]), __float_as_uint(v[4 * j + 3]));
+            __syncwarp();
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {  // 4 rows x 128 bytes per instruction
-                    const int r = 4 * i + (lane >> 3), c = lane & 7;
-                    if (m0w + r < a.M)
-                        *reinterpret_cast<uint4 *>(d32 + (int64_t)(m0w + r) * a.d_sm + nb + 4 * c) = *tile32(tf, r, c);
-                }
-                __syncwarp();
+            for (int i = 0; i < 8; ++i) {  // 4 rows x 128 bytes per instruction
+                const int r = 4 * i + (lane >> 3), c = lane & 7;
+                if (m0w + r < a.M)
+                    *reinterpret_cast<uint4 *>(out + (int64_t)(m0w + r) * a.d_sm + nb + 4 * c) = *tile32(tf, r, c);
             }
-            if (a.epi == EPI_SILU && a.Z16) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    *tile16(tz, lane, j) =
-                        make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
-                                   pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
-                tile16_store(tz, a.Z16, a.d_sm, m0w, a.M, nb);
-            }
-            if (a.D16) {
-                if (a.epi == EPI_SILU) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = silu(v[i]);
-                } else if (a.epi == EPI_DSILU) {
-                    // the pre-activations of the warp's rows, loaded whole rows at a time
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int r = 8 * i + (lane >> 2), c = lane & 3;
-                        if (m0w + r < a.M)
-                            *tile16(tz, r, c) =
-                                *reinterpret_cast<const uint4 *>(a.Zin + (int64_t)(m0w + r) * a.d_sm + nb + 8 * c);
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint4 zq = *tile16(tz, lane, j);
-                        const uint32_t zw[4] = {zq.x, zq.y, zq.z, zq.w};
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const __nv_bfloat162 z2 = *reinterpret_cast<const __nv_bfloat162 *>(&zw[q]);
-                            v[8 * j + 2 * q] *= dsilu(__low2float(z2));
-                            v[8 * j + 2 * q + 1] *= dsilu(__high2float(z2));
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    *tile16(th, lane, j) =
-                        make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
-                                   pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
-                tile16_store(th, a.D16, a.d_sm, m0w, a.M, nb);
-            }
+            __syncwarp();
         } else if (m < a.M) {
-            const int64_t o = (int64_t)m * a.d_sm + nb;
-            float *d32 = a.D32 ? a.D32 + (int64_t)blockIdx.z * a.M * a.d_sm + o : nullptr;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {  // unrolled: v stays in registers
                 if (i >= nn) break;
-                const float z = v[i];
-                if (d32) d32[i] = z;
-                if (a.epi == EPI_SILU && a.Z16) a.Z16[o + i] = __float2bfloat16(z);
-                if (a.D16) {
-                    float h = z;
-                    if (a.epi == EPI_SILU) h = silu(z);
-                    else if (a.epi == EPI_DSILU) h = z * dsilu(__bfloat162float(a.Zin[o + i]));
-                    a.D16[o + i] = __float2bfloat16(h);
-                }
+                out[(int64_t)m * a.d_sm + nb + i] = v[i];
             }
         }
     }
@@ -585,155 +516,24 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NT));
 }
 
-// out[i] = sum over z of part[z][i] (fixed order), optional BF16 copy.
-__global__ void k_sum_splits(const float *part, int splits, int64_t n, float *out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(int64_t)z * n + i];
-    out[i] = s;
-}
-
 }  // namespace
 
-namespace {
-
-constexpr int kWidth = 256;
-constexpr int kFeat = 128;       // Fourier features, padded
-constexpr int kFreq = 15;
-constexpr int kIn = 4, kOut = 4;
-constexpr int kHidden = 5;       // layers with SiLU
-constexpr int kSplitRows = 256;  // batch rows per split of a weight-gradient GEMM (16384 rows: 128 CTAs)
-
-// Fourier features of x[b][4] (inputs normalised to [-1, 1]).
-__global__ void k_features(const float *x, int B, bf16 *f) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    bf16 *o = f + (int64_t)b * kFeat;
-    int q = 0;
-    for (int i = 0; i < kIn; ++i) {
-        const float v = x[(int64_t)b * kIn + i];
-        o[q++] = __float2bfloat16(v);
-        float w = 3.14159265358979f;
-        for (int j = 0; j < kFreq; ++j, w *= 2.0f) {
-            o[q++] = __float2bfloat16(sinf(w * v));
-            o[q++] = __float2bfloat16(cosf(w * v));
-        }
-    }
-    for (; q < kFeat; ++q) o[q] = __float2bfloat16(0.0f);
-}
-
-// Output layer y = W6 h5 + b6 on CUDA cores (4 outputs), and for training
-// dy = 2 (y - t) / (4 B) plus per-block partial sums of (y - t)^2.
-__global__ void k_output(const bf16 *h, const float *W6, const float *b6, int B, float *y, const float *t,
-                         float *dy, float *loss_part) {
-    __shared__ float red[8];
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (b < B) {
-        float acc[kOut];
-        for (int o = 0; o < kOut; ++o) acc[o] = b6[o];
-        const bf16 *hr = h + (int64_t)b * kWidth;
-        for (int j = 0; j < kWidth; ++j) {
-            const float hv = __bfloat162float(hr[j]);
-            for (int o = 0; o < kOut; ++o) acc[o] += W6[o * kWidth + j] * hv;
-        }
-        for (int o = 0; o < kOut; ++o) {
-            if (y) y[(int64_t)b * kOut + o] = acc[o];
-            if (t) {
-                const float d = acc[o] - t[(int64_t)b * kOut + o];
-                l += d * d;
-                dy[(int64_t)b * kOut + o] = 2.0f * d / (float)(kOut * B);
-            }
-        }
-    }
-    if (!loss_part) return;
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.0f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-        loss_part[blockIdx.x] = s;
-    }
-}
-
-// dz5 = (dy W6) * silu'(z5), BF16.
-__global__ void k_output_back(const float *dy, const float *W6, const bf16 *z5, int B, bf16 *dz) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)B * kWidth) return;
-    const int b = (int)(i / kWidth), j = (int)(i % kWidth);
-    float s = 0.0f;
-    for (int o = 0; o < kOut; ++o) s += dy[(int64_t)b * kOut + o] * W6[o * kWidth + j];
-    dz[i] = __float2bfloat16(s * dsilu(__bfloat162float(z5[i])));
-}
-
-// Gradient of the output layer: part[chunk][o * 256 + j] = sum over the chunk's
-// rows of dy[b][o] h5[b][j]; part[chunk][1024 + o] = sum of dy[b][o].
-__global__ void k_output_wgrad(const float *dy, const bf16 *h, int B, int rows, float *part) {
-    const int chunk = blockIdx.x, idx = blockIdx.y * blockDim.x + threadIdx.x;
-    if (idx >= kOut * kWidth + kOut) return;
-    const int b0 = chunk * rows, b1 = min(B, b0 + rows);
-    float s = 0.0f;
-    if (idx < kOut * kWidth) {
-        const int o = idx / kWidth, j = idx % kWidth;
-        for (int b = b0; b < b1; ++b) s += dy[(int64_t)b * kOut + o] * __bfloat162float(h[(int64_t)b * kWidth + j]);
-    } else {
-        const int o = idx - kOut * kWidth;
-        for (int b = b0; b < b1; ++b) s += dy[(int64_t)b * kOut + o];
-    }
-    part[(int64_t)chunk * (kOut * kWidth + kOut) + idx] = s;
-}
-
-// Column sums of dz [B][256] over row chunks: part[chunk][j].
-__global__ void k_colsum(const bf16 *dz, int B, int rows, float *part) {
-    const int chunk = blockIdx.x, j = threadIdx.x;
-    const int b0 = chunk * rows, b1 = min(B, b0 + rows);
-    float s = 0.0f;
-    for (int b = b0; b < b1; ++b) s += __bfloat162float(dz[(int64_t)b * kWidth + j]);
-    part[(int64_t)chunk * kWidth + j] = s;
-}
-
-// Adam (Kingma & Ba, 2015) on the FP32 master parameters; refreshes the BF16
-// copies of the tensor-core weights (entries with wmap[i] >= 0).
-__global__ void k_adam(float *p, const float *g, float *m, float *v, int64_t n, float lr, float b1, float b2,
-                       float eps, float c1, float c2, const int64_t *wmap, bf16 *wbf) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    p[i] = pi;
-    if (wmap[i] >= 0) wbf[wmap[i]] = __float2bfloat16(pi);
-}
-
-__global__ void k_to_bf16(const float *p, int64_t n, const int64_t *wmap, bf16 *wbf) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && wmap[i] >= 0) wbf[wmap[i]] = __float2bfloat16(p[i]);
-}
-
-}  // namespace
+#include "mlp_net.cuh"
 
 using namespace psst;
 
 struct psst_mlp {
-    int device = 0;
+    int device = 0, sms = 1;
     cudaStream_t own = nullptr, stream = nullptr;
-    int64_t nparam = 0, nwbf = 0;
-    int64_t offW[6] = {}, offb[6] = {}, offWbf[5] = {};
-    int din[6] = {kFeat, kWidth, kWidth, kWidth, kWidth, kWidth}, dout[6] = {kWidth, kWidth, kWidth, kWidth, kWidth, kOut};
+    NetLayout net{};
     float *p = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;
-    int64_t *wmap = nullptr;
     bf16 *wbf = nullptr;
     int64_t step = 0;
-    int cap = 0;
-    bf16 *F = nullptr, *Z[kHidden] = {}, *H[kHidden] = {}, *dZ[2] = {};
-    float *y = nullptr, *dy = nullptr, *lpart = nullptr, *part = nullptr;
-    int64_t part_n = 0;
-    int *err = nullptr;
+    int cap = 0, map_rows = 0;  // rows of the training workspace; rows that its tensor maps end at
+    bf16 *F = nullptr, *Z[kHidden - 1] = {}, *H[kHidden] = {}, *dZ[kHidden] = {};
+    float *dy = nullptr, *lpart = nullptr, *part = nullptr;
+    NetMaps maps{};
+    int *status = nullptr;  // error word, loss
     std::vector<void *> allocs, ws;
     ~psst_mlp() {
         cudaSetDevice(device);
@@ -840,7 +640,7 @@ GemmPlan plan(const GemmArgs &a0, int splits) {
     GemmPlan p;
     p.a = a0;
     GemmArgs &a = p.a;
-    a.vec = a.d_sm % 8 == 0 && aligned16(a.D32) && aligned16(a.D16) && aligned16(a.Z16) && aligned16(a.Zin);
+    a.vec = a.d_sm % 4 == 0 && aligned16(a.D32);
     p.nt = NT;
     p.grid = dim3((a.M + kTileM - 1) / kTileM, (a.N + NT - 1) / NT, splits);
     // TMA boxes are whole 64-wide chunks: a split range must be whole chunks unless it is the only one
@@ -875,11 +675,6 @@ void launch(const GemmPlan &p, cudaStream_t s) {
         launch_nt<256>(p, s);
 }
 
-template <int NT>
-void gemm(const GemmArgs &a, int splits, cudaStream_t s) {
-    launch(plan<NT>(a, splits), s);
-}
-
 GemmArgs gargs(const bf16 *A, int64_t a_sm, int64_t a_sk, const bf16 *B, int64_t b_sn, int64_t b_sk, int M, int N,
                int K, int *err) {
     GemmArgs a{};
@@ -900,103 +695,114 @@ GemmArgs gargs(const bf16 *A, int64_t a_sm, int64_t a_sk, const bf16 *B, int64_t
 
 unsigned nb(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
-void ensure_ws(psst_mlp *m, int B) {
-    if (B <= m->cap) return;
-    for (void *q : m->ws) cudaFree(q);
-    m->ws.clear();
-    const int cap = std::max(B, 2 * m->cap);
-    m->F = dmalloc<bf16>(m->ws, (size_t)cap * kFeat);
-    for (int l = 0; l < kHidden; ++l) {
-        m->Z[l] = dmalloc<bf16>(m->ws, (size_t)cap * kWidth);
-        m->H[l] = dmalloc<bf16>(m->ws, (size_t)cap * kWidth);
-    }
-    m->dZ[0] = dmalloc<bf16>(m->ws, (size_t)cap * kWidth);
-    m->dZ[1] = dmalloc<bf16>(m->ws, (size_t)cap * kWidth);
-    m->y = dmalloc<float>(m->ws, (size_t)cap * kOut);
-    m->dy = dmalloc<float>(m->ws, (size_t)cap * kOut);
-    m->lpart = dmalloc<float>(m->ws, nb(cap));
-    const int64_t splits = (cap + kSplitRows - 1) / kSplitRows;
-    m->part_n = splits * (int64_t)kWidth * kWidth;
-    m->part = dmalloc<float>(m->ws, m->part_n);
-    m->cap = cap;
+// Box 64 x 64 of a row-major [rows][cols] BF16 matrix, 128-byte swizzle.
+CUtensorMap box_map(const bf16 *g, int rows, int cols) { return operand_map(g, cols, 1, rows, cols, 64); }
+
+// Partial sums of one layer's weights: parameters [out][in] from `first` on, `splits`
+// times nparam apart; boxes of 32 x 32, 128-byte swizzle.
+CUtensorMap part_map(const float *first, int in, int splits, int nparam) {
+    CUtensorMap map;
+    const cuuint64_t dim[3] = {(cuuint64_t)in, (cuuint64_t)kWidth, (cuuint64_t)splits};
+    const cuuint64_t stride[2] = {(cuuint64_t)in * 4, (cuuint64_t)nparam * 4};
+    const cuuint32_t box[3] = {32, 32, 1}, estride[3] = {1, 1, 1};
+    const CUresult r = encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(first), dim, stride,
+                                      box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) raise(PSST_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+    return map;
 }
 
-void check_err(psst_mlp *m) {
-    int e = 0;
-    ck(cudaMemcpyAsync(&e, m->err, sizeof e, cudaMemcpyDeviceToHost, m->stream), "error word");
+// Training workspace and tensor maps for batches of B rows. The maps end at row
+// B: rows past it read as zeros and are not written.
+void ensure_ws(psst_mlp *m, int B) {
+    if (B > m->cap) {
+        for (void *q : m->ws) cudaFree(q);
+        m->ws.clear();
+        const int cap = std::max(B, 2 * m->cap);
+        m->cap = m->map_rows = 0;
+        const int splits = std::min((int)nb(cap, kSplitRows), kSplitsMax);
+        size_t off = 0;  // one allocation
+        auto take = [&](size_t bytes) {
+            const size_t at = off;
+            off += (bytes + 255) / 256 * 256;
+            return at;
+        };
+        const size_t o_f = take((size_t)cap * kFeat * sizeof(bf16));
+        size_t o_h[kHidden], o_dz[kHidden], o_z[kHidden - 1];
+        for (int l = 0; l < kHidden; ++l) {
+            o_h[l] = take((size_t)cap * kWidth * sizeof(bf16));
+            o_dz[l] = take((size_t)cap * kWidth * sizeof(bf16));
+            if (l + 1 < kHidden) o_z[l] = take((size_t)cap * kWidth * sizeof(bf16));
+        }
+        const size_t o_dy = take((size_t)cap * kOut * sizeof(float)), o_loss = take(nb(cap, kTileM) * sizeof(float)),
+                     o_part = take((size_t)splits * m->net.nparam * sizeof(float));
+        unsigned char *base = dmalloc<unsigned char>(m->ws, off);
+        m->F = (bf16 *)(base + o_f);
+        for (int l = 0; l < kHidden; ++l) {
+            m->H[l] = (bf16 *)(base + o_h[l]);
+            m->dZ[l] = (bf16 *)(base + o_dz[l]);
+            if (l + 1 < kHidden) m->Z[l] = (bf16 *)(base + o_z[l]);
+        }
+        m->dy = (float *)(base + o_dy);
+        m->lpart = (float *)(base + o_loss);
+        m->part = (float *)(base + o_part);
+        for (int l = 0; l < kHidden; ++l)
+            m->maps.part[l] = part_map(m->part + m->net.offW[l], net_din(l), splits, m->net.nparam);
+        m->cap = cap;
+    }
+    if (B != m->map_rows) {
+        m->maps.f = box_map(m->F, B, kFeat);
+        for (int l = 0; l < kHidden; ++l) {
+            m->maps.h[l] = box_map(m->H[l], B, kWidth);
+            m->maps.dz[l] = box_map(m->dZ[l], B, kWidth);
+            if (l + 1 < kHidden) m->maps.z[l] = box_map(m->Z[l], B, kWidth);
+        }
+        m->map_rows = B;
+    }
+}
+
+// The error word (and the loss after a training pass), once the stream's work is done.
+float finish(psst_mlp *m) {
+    ck(cudaGetLastError(), "network launch");
+    int status[2];
+    ck(cudaMemcpyAsync(status, m->status, sizeof status, cudaMemcpyDeviceToHost, m->stream), "status");
     ck(cudaStreamSynchronize(m->stream), "stream sync");
-    if (e) {
-        ck(cudaMemsetAsync(m->err, 0, sizeof(int), m->stream), "memset");
+    if (status[0]) {
+        ck(cudaMemsetAsync(m->status, 0, sizeof(int), m->stream), "memset");
         raise(PSST_ERR_TIMEOUT, "tensor-core GEMM: an mbarrier wait ran out");
     }
+    float loss;
+    std::memcpy(&loss, status + 1, sizeof loss);
+    return loss;
 }
 
-// Forward pass; with t != null also the loss terms (returns the loss).
-float forward(psst_mlp *m, const float *x, int B, const float *t, float *yout) {
-    cudaStream_t s = m->stream;
-    k_features<<<nb(B), 256, 0, s>>>(x, B, m->F);
-    const bf16 *in = m->F;
-    int64_t ld = kFeat;
-    for (int l = 0; l < kHidden; ++l) {
-        GemmArgs a = gargs(in, ld, 1, m->wbf + m->offWbf[l], ld, 1, B, kWidth, (int)ld, m->err);
-        a.bias = m->p + m->offb[l];
-        a.epi = EPI_SILU;
-        a.Z16 = m->Z[l];
-        a.D16 = m->H[l];
-        a.d_sm = kWidth;
-        gemm<256>(a, 1, s);
-        in = m->H[l];
-        ld = kWidth;
-    }
-    k_output<<<nb(B), 256, 0, s>>>(m->H[kHidden - 1], m->p + m->offW[5], m->p + m->offb[5], B, yout ? yout : m->y, t,
-                                   m->dy, t ? m->lpart : nullptr);
-    ck(cudaGetLastError(), "forward");
-    if (!t) return 0.0f;
-    std::vector<float> lp(nb(B));
-    ck(cudaMemcpyAsync(lp.data(), m->lpart, lp.size() * sizeof(float), cudaMemcpyDeviceToHost, s), "loss copy");
-    check_err(m);
-    double sum = 0.0;
-    for (float v : lp) sum += v;
-    return (float)(sum / ((double)kOut * B));
+template <bool TRAIN>
+void chain(psst_mlp *m, const float *x, const float *t, int B, float *y) {
+    static thread_local unsigned long long done_devices = 0;
+    smem_attribute(k_net<TRAIN>, net_smem<TRAIN>(), done_devices);
+    k_net<TRAIN><<<nb(B, kTileM), kNetThreads, net_smem<TRAIN>(), m->stream>>>(
+        m->maps, NetArgs{m->net, m->p, x, t, y, m->dy, m->lpart, B, m->status});
 }
 
-// Gradients of the loss of the last forward pass into m->g.
-void backward(psst_mlp *m, int B) {
+// Forward and backward pass, weight gradients, and their sums over the batch:
+// into m->g (adam null) or straight into an Adam update.
+void gradients(psst_mlp *m, const float *x, const float *t, int B, const AdamArgs *adam) {
     cudaStream_t s = m->stream;
-    const int splits = (B + kSplitRows - 1) / kSplitRows;
-    // output layer (CUDA cores)
-    k_output_back<<<nb((int64_t)B * kWidth), 256, 0, s>>>(m->dy, m->p + m->offW[5], m->Z[kHidden - 1], B, m->dZ[0]);
-    const int nout = kOut * kWidth + kOut;
-    k_output_wgrad<<<dim3(splits, nb(nout)), 256, 0, s>>>(m->dy, m->H[kHidden - 1], B, kSplitRows, m->part);
-    k_sum_splits<<<nb(nout), 256, 0, s>>>(m->part, splits, nout, m->g + m->offW[5]);
-    int cur = 0;
-    for (int l = kHidden - 1; l >= 0; --l) {
-        const bf16 *prev = l == 0 ? m->F : m->H[l - 1];
-        const int din = m->din[l];
-        // dW_l = dZ_l^T . H_{l-1}: split over batch rows, fixed-order sum
-        GemmArgs a = gargs(m->dZ[cur], 1, kWidth, prev, 1, din, kWidth, din, B, m->err);
-        a.k_split = kSplitRows;
-        a.D32 = m->part;
-        a.d_sm = din;
-        if (din == 256)
-            gemm<256>(a, splits, s);
+    chain<true>(m, x, t, B, nullptr);
+    static thread_local unsigned long long done_devices = 0;
+    smem_attribute(k_wgrad, kWgradSmem, done_devices);
+    const int splits = (int)nb(B, kSplitRows), n4 = (int)(m->net.nparam / 4);
+    for (int s0 = 0; s0 < splits; s0 += kSplitsMax) {
+        const int n = std::min(splits - s0, kSplitsMax);
+        const int units = n * kWgradUnits;
+        k_wgrad<<<std::min(units, m->sms), kWgradThreads, kWgradSmem, s>>>(
+            m->maps, WgradArgs{m->net, m->dy, m->part, B, s0, units, m->status});
+        const LossArgs loss{m->lpart, (int)nb(B, kTileM), 1.0 / ((double)kOut * B), m->status};
+        if (adam && s0 + n == splits)
+            k_reduce<true><<<nb(n4), 256, 0, s>>>(m->part, n, n4, s0 == 0, m->g, *adam, loss);
         else
-            gemm<128>(a, splits, s);
-        k_sum_splits<<<nb((int64_t)kWidth * din), 256, 0, s>>>(m->part, splits, (int64_t)kWidth * din,
-                                                               m->g + m->offW[l]);
-        k_colsum<<<splits, kWidth, 0, s>>>(m->dZ[cur], B, kSplitRows, m->part);
-        k_sum_splits<<<1, kWidth, 0, s>>>(m->part, splits, kWidth, m->g + m->offb[l]);
-        if (l > 0) {  // dZ_{l-1} = (dZ_l . W_l) * silu'(Z_{l-1})
-            GemmArgs d = gargs(m->dZ[cur], kWidth, 1, m->wbf + m->offWbf[l], 1, din, B, kWidth, kWidth, m->err);
-            d.epi = EPI_DSILU;
-            d.Zin = m->Z[l - 1];
-            d.D16 = m->dZ[cur ^ 1];
-            d.d_sm = kWidth;
-            gemm<256>(d, 1, s);
-            cur ^= 1;
-        }
+            k_reduce<false><<<nb(n4), 256, 0, s>>>(m->part, n, n4, s0 == 0, m->g, AdamArgs{}, loss);
     }
-    ck(cudaGetLastError(), "backward");
 }
 
 }  // namespace
@@ -1026,22 +832,11 @@ extern "C" psst_status psst_mlp_create(int device, uint64_t seed, psst_mlp **out
     ck(cudaSetDevice(device), "cudaSetDevice");
     ck(cudaStreamCreateWithFlags(&m->own, cudaStreamNonBlocking), "stream");
     m->stream = m->own;
-    int64_t off = 0, wo = 0;
-    for (int l = 0; l < 6; ++l) {
-        m->offW[l] = off;
-        off += (int64_t)m->dout[l] * m->din[l];
-        m->offb[l] = off;
-        off += m->dout[l];
-        if (l < kHidden) {
-            m->offWbf[l] = wo;
-            wo += (int64_t)m->dout[l] * m->din[l];
-        }
-    }
-    m->nparam = off;
-    m->nwbf = wo;
+    m->net = net_layout();
+    ck(cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, device), "device attribute");
+    const int off = m->net.nparam;
     // PyTorch's default Linear initialisation: U(-1/sqrt(in), 1/sqrt(in)) for weights and biases
     std::vector<float> h(off);
-    std::vector<int64_t> map(off, -1);
     uint64_t st = seed * 0x9E3779B97F4A7C15ull + 0x2545F4914F6CDD1Dull;
     auto uni = [&]() {  // splitmix64 -> [0, 1)
         st += 0x9E3779B97F4A7C15ull;
@@ -1052,35 +847,33 @@ extern "C" psst_status psst_mlp_create(int device, uint64_t seed, psst_mlp **out
         return (double)(z >> 11) * (1.0 / 9007199254740992.0);
     };
     for (int l = 0; l < 6; ++l) {
-        const double bound = 1.0 / std::sqrt((double)(l == 0 ? 4 * (2 * kFreq + 1) : m->din[l]));
-        for (int64_t i = m->offW[l]; i < m->offb[l] + m->dout[l]; ++i) h[i] = (float)((2.0 * uni() - 1.0) * bound);
-        if (l < kHidden)
-            for (int64_t i = 0; i < (int64_t)m->dout[l] * m->din[l]; ++i) map[m->offW[l] + i] = m->offWbf[l] + i;
+        const double bound = 1.0 / std::sqrt((double)(l == 0 ? 4 * (2 * kFreq + 1) : kWidth));
+        const int end = m->net.offb[l] + (l < kHidden ? kWidth : kOut);
+        for (int i = m->net.offW[l]; i < end; ++i) h[i] = (float)((2.0 * uni() - 1.0) * bound);
     }
     m->p = dmalloc<float>(m->allocs, off);
     m->g = dmalloc<float>(m->allocs, off);
     m->m1 = dmalloc<float>(m->allocs, off);
     m->m2 = dmalloc<float>(m->allocs, off);
-    m->wmap = dmalloc<int64_t>(m->allocs, off);
-    m->wbf = dmalloc<bf16>(m->allocs, wo);
-    m->err = dmalloc<int>(m->allocs, 1);
+    m->wbf = dmalloc<bf16>(m->allocs, m->net.nwbf);
+    m->status = dmalloc<int>(m->allocs, 2);
+    for (int l = 0; l < kHidden; ++l) m->maps.w[l] = box_map(m->wbf + m->net.offWbf[l], kWidth, net_din(l));
     ck(cudaMemcpy(m->p, h.data(), off * sizeof(float), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(m->wmap, map.data(), off * sizeof(int64_t), cudaMemcpyHostToDevice), "upload");
     ck(cudaMemset(m->m1, 0, off * sizeof(float)), "memset");
     ck(cudaMemset(m->m2, 0, off * sizeof(float)), "memset");
     ck(cudaMemset(m->g, 0, off * sizeof(float)), "memset");
-    ck(cudaMemset(m->err, 0, sizeof(int)), "memset");
-    k_to_bf16<<<nb(off), 256, 0, m->stream>>>(m->p, off, m->wmap, m->wbf);
+    ck(cudaMemset(m->status, 0, 2 * sizeof(int)), "memset");
+    k_to_bf16<<<nb(off / 4), 256, 0, m->stream>>>(m->p, m->net, m->wbf);
     ck(cudaStreamSynchronize(m->stream), "init");
     *out = m.release();
     MLP_END
 }
 
-extern "C" int64_t psst_mlp_param_count(const psst_mlp *m) { return m ? m->nparam : -1; }
+extern "C" int64_t psst_mlp_param_count(const psst_mlp *m) { return m ? m->net.nparam : -1; }
 
 extern "C" psst_status psst_mlp_get_params(psst_mlp *m, float *out, int64_t n) {
     MLP_BEGIN
-    if (!m || !out || n != m->nparam) raise(PSST_ERR_ARG, "psst_mlp_get_params: bad argument");
+    if (!m || !out || n != m->net.nparam) raise(PSST_ERR_ARG, "psst_mlp_get_params: bad argument");
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     ck(cudaMemcpyAsync(out, m->p, n * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "copy");
     ck(cudaStreamSynchronize(m->stream), "sync");
@@ -1089,10 +882,10 @@ extern "C" psst_status psst_mlp_get_params(psst_mlp *m, float *out, int64_t n) {
 
 extern "C" psst_status psst_mlp_set_params(psst_mlp *m, const float *in, int64_t n) {
     MLP_BEGIN
-    if (!m || !in || n != m->nparam) raise(PSST_ERR_ARG, "psst_mlp_set_params: bad argument");
+    if (!m || !in || n != m->net.nparam) raise(PSST_ERR_ARG, "psst_mlp_set_params: bad argument");
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     ck(cudaMemcpyAsync(m->p, in, n * sizeof(float), cudaMemcpyHostToDevice, m->stream), "copy");
-    k_to_bf16<<<nb(n), 256, 0, m->stream>>>(m->p, n, m->wmap, m->wbf);
+    k_to_bf16<<<nb(n / 4), 256, 0, m->stream>>>(m->p, m->net, m->wbf);
     ck(cudaStreamSynchronize(m->stream), "sync");
     m->step = 0;
     ck(cudaMemset(m->m1, 0, n * sizeof(float)), "memset");
@@ -1104,9 +897,8 @@ extern "C" psst_status psst_mlp_forward(psst_mlp *m, const float *x, int B, floa
     MLP_BEGIN
     if (!m || !x || !y || B <= 0) raise(PSST_ERR_ARG, "psst_mlp_forward: bad argument");
     ck(cudaSetDevice(m->device), "cudaSetDevice");
-    ensure_ws(m, B);
-    forward(m, x, B, nullptr, y);
-    check_err(m);
+    chain<false>(m, x, nullptr, B, y);
+    finish(m);
     MLP_END
 }
 
@@ -1116,10 +908,9 @@ extern "C" psst_status psst_mlp_gradients(psst_mlp *m, const float *x, const flo
     if (!m || !x || !t || B <= 0) raise(PSST_ERR_ARG, "psst_mlp_gradients: bad argument");
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     ensure_ws(m, B);
-    const float l = forward(m, x, B, t, nullptr);
-    backward(m, B);
-    if (grads) ck(cudaMemcpyAsync(grads, m->g, m->nparam * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "copy");
-    check_err(m);
+    gradients(m, x, t, B, nullptr);
+    const float l = finish(m);
+    if (grads) ck(cudaMemcpy(grads, m->g, m->net.nparam * sizeof(float), cudaMemcpyDeviceToHost), "copy");
     if (loss) *loss = l;
     MLP_END
 }
@@ -1130,16 +921,13 @@ extern "C" psst_status psst_mlp_train_step(psst_mlp *m, const float *x, const fl
     if (!m || !x || !t || B <= 0) raise(PSST_ERR_ARG, "psst_mlp_train_step: bad argument");
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     ensure_ws(m, B);
-    const float l = forward(m, x, B, t, nullptr);
-    backward(m, B);
-    m->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = (float)(1.0 - std::pow((double)b1, (double)m->step));
-    const float c2 = (float)(1.0 - std::pow((double)b2, (double)m->step));
-    k_adam<<<nb(m->nparam), 256, 0, m->stream>>>(m->p, m->g, m->m1, m->m2, m->nparam, lr, b1, b2, 1e-8f, c1, c2,
-                                                  m->wmap, m->wbf);
-    ck(cudaGetLastError(), "adam");
-    check_err(m);
+    const float c1 = (float)(1.0 - std::pow((double)b1, (double)(m->step + 1)));
+    const float c2 = (float)(1.0 - std::pow((double)b2, (double)(m->step + 1)));
+    const AdamArgs adam{m->net, m->p, m->m1, m->m2, m->wbf, lr, b1, b2, 1e-8f, c1, c2};
+    gradients(m, x, t, B, &adam);
+    const float l = finish(m);
+    m->step += 1;
     if (loss) *loss = l;
     MLP_END
 }
