@@ -40,6 +40,27 @@ struct alignas(16) FaceRec {
     R o1[DIM];
 };
 
+// What the face pass reads of the face records, packed for it: the neighbours,
+// area, normal and the offsets that the reconstruction REC uses, each rounded to R
+// as the pass rounds it. N bytes a face, split into columns of 32, 16, 8 and 4
+// bytes (each [nface], coalesced, 256-byte aligned). 3D FP32: 48 bytes for MUSCL
+// and 36 for Darwish-Moukalled instead of the record's 64; FP64: 88 and 64 instead
+// of 96.
+template <typename R, int DIM, int REC>
+struct FaceCols {
+    static constexpr int NR = 1 + DIM + (REC >= 1 ? DIM : 0) + (REC == 2 ? DIM : 0);  // values after c0, c1
+    static constexpr int N = 8 + NR * (int)sizeof(R);
+    // bytes in front of byte B of the first nface faces' columns
+    static constexpr int64_t column(int64_t nface, int B) { return B == 0 ? 0 : pad(nface, 32) * (B / 32) + tail(nface, B); }
+    static constexpr int64_t bytes(int64_t nface) { return column(nface, N) + 256; }
+
+   private:
+    static constexpr int64_t pad(int64_t nface, int w) { return (nface * w + 255) / 256 * 256; }
+    static constexpr int64_t tail(int64_t nface, int B) {
+        return (B & 16 ? pad(nface, 16) : 0) + (B & 8 ? pad(nface, 8) : 0) + (B & 4 ? pad(nface, 4) : 0);
+    }
+};
+
 // Output of the face pass for one face: flux * area (DIM+2), then the face's
 // local-time-step terms: for LocalAccTime1 the two neighbours' normal
 // velocities and the mean sound speed (the face area comes from
@@ -68,6 +89,7 @@ struct DevGrid {
     int32_t nface;    // active faces (zone 31 excluded); interior faces first
     int32_t nfi;      // interior faces: device ids [0, nfi)
     const void *frec;         // [nface] FaceRec<R, DIM>
+    const char *fcols;        // the part of it that the face pass reads, by columns (FaceCols)
     const double *beta;       // [nface] Green-Gauss interpolation weight (reference table)
     const double *V;          // [nint] cell volume
     const double *xc;         // [dim][nall] centroid (ghost: its face centre); least squares only
@@ -77,6 +99,7 @@ struct DevGrid {
     const int32_t *csr_nb;    // the cell across each csr_ent face (saves a dependent load)
     const void *csr_s;        // R per csr_ent: the face's area, rounded to R (LocalAccTime1)
     const uint64_t *wperm;    // [nint] 4-bit slots: k-th face of the cell's own face order
+    int32_t same_order;       // every cell's own face order is the face-loop order
     const double *lsq_r;      // [3 (2D) or 7 (3D)][nint] least-squares coefficients (reference table)
     const double *vk_eps2;    // [nint] Venkatakrishnan epsilon^2 = (K h)^3, h = V^(1/dim)
     // Green-Gauss on meshes of 4 faces per cell (tets, quads), else null; per
@@ -116,7 +139,7 @@ struct DevState {
 
 template <typename R>
 struct DevWork {
-    double *w, *pw;      // [dim+2][nint] conservative state, previous-stage state
+    double *w, *pw;      // [dim+2][nint] conservative state; its value at stage 1 (stage-by-stage API)
     void *grec;          // [nint] GradRec<R, DIM>
     void *fout;          // [nface] FaceOut<R, DIM>, written by the face pass
     R *res;              // [dim+2][nint] residual (stage-by-stage API only)

@@ -21,16 +21,18 @@
 #include <cstddef>
 #include <cstdint>
 
+#include <type_traits>
+
 #include "devgrid.hpp"
 
 // Register budgets of the three hot kernels on the FP32 path (compile-time
-// tuning; the values are the measured best on the 6M-tet benchmark): k_face
-// register cap, k_cell and k_gradient minimum resident 256-thread blocks per
-// SM (gradient: 3, room for the pipelined loop's next-face records). The
-// FP64 instantiations (twice the registers per value) get budgets that do
-// not spill.
+// tuning; the values are the measured best, 3D: k_face register cap (64 with the
+// straight-line flux: 43.4 us on 750k tets, 44.5 at 56; 48 in 2D and with the
+// branching one), k_cell and k_gradient minimum resident 256-thread blocks per SM
+// (gradient: 4 in 3D, 40.1 -> 38.2 us on 750k tets; 3 in 2D). The FP64
+// instantiations (twice the registers per value) get budgets that do not spill.
 #ifndef PSST_FACE_MAXNREG
-#define PSST_FACE_MAXNREG 48
+#define PSST_FACE_MAXNREG 64
 #endif
 #ifndef PSST_FACE_MAXNREG_DM  // the DM reconstruction holds both neighbours' projections
 #define PSST_FACE_MAXNREG_DM 56
@@ -39,7 +41,7 @@
 #define PSST_CELL_MINB 4
 #endif
 #ifndef PSST_GRAD_MINB
-#define PSST_GRAD_MINB 3
+#define PSST_GRAD_MINB 4
 #endif
 #define PSST_BUDGET(R, f32, f64) (sizeof(R) == 8 ? (f64) : (f32))
 #ifndef PSST_GRAD_PIPE
@@ -128,6 +130,62 @@ __device__ __forceinline__ void face_offsets(const FaceRec<R, DIM> *p, int side,
         off[k] = side ? x1 : x0;
     }
 }
+
+// Face f of FaceCols<R, DIM, REC>: the packed 4-byte words, one load per column.
+template <typename R, int DIM, int REC>
+struct PackedFace {
+    static constexpr int NW = FaceCols<R, DIM, REC>::N / 4;
+    uint32_t w[NW];
+    __device__ __forceinline__ R value(int i) const {  // i-th R after the neighbours
+        if constexpr (sizeof(R) == 8)
+            return __hiloint2double((int)w[3 + 2 * i], (int)w[2 + 2 * i]);
+        else
+            return __uint_as_float(w[2 + i]);
+    }
+    __device__ __forceinline__ void put(int i, R x) {
+        if constexpr (sizeof(R) == 8) {
+            w[2 + 2 * i] = (uint32_t)__double2loint(x);
+            w[3 + 2 * i] = (uint32_t)__double2hiint(x);
+        } else {
+            w[2 + i] = __float_as_uint(x);
+        }
+    }
+    // each column of the face, as f(its address, first word, words)
+    template <class F>
+    static __device__ __forceinline__ void columns(char *base, int64_t nface, int64_t face, F f) {
+        using C = FaceCols<R, DIM, REC>;
+#pragma unroll
+        for (int b = 0; b + 32 <= C::N; b += 32) f(base + C::column(nface, b) + face * 32, b / 4, std::integral_constant<int, 8>());
+        constexpr int B16 = C::N & ~31, B8 = C::N & ~15, B4 = C::N & ~7;
+        if constexpr (C::N & 16) f(base + C::column(nface, B16) + face * 16, B16 / 4, std::integral_constant<int, 4>());
+        if constexpr (C::N & 8) f(base + C::column(nface, B8) + face * 8, B8 / 4, std::integral_constant<int, 2>());
+        if constexpr (C::N & 4) f(base + C::column(nface, B4) + face * 4, B4 / 4, std::integral_constant<int, 1>());
+    }
+    __device__ __forceinline__ void load(const char *base, int64_t nface, int64_t face) {
+        columns(const_cast<char *>(base), nface, face, [&](const char *p, int i, auto words) {
+            constexpr int W = decltype(words)::value;
+            if constexpr (W == 8)
+                asm("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                    : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3]), "=r"(w[i + 4]), "=r"(w[i + 5]),
+                      "=r"(w[i + 6]), "=r"(w[i + 7])
+                    : "l"(p));
+            else if constexpr (W == 4)
+                asm("ld.global.v4.b32 {%0,%1,%2,%3}, [%4];"
+                    : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3])
+                    : "l"(p));
+            else if constexpr (W == 2)
+                asm("ld.global.v2.b32 {%0,%1}, [%2];" : "=r"(w[i]), "=r"(w[i + 1]) : "l"(p));
+            else
+                asm("ld.global.b32 %0, [%1];" : "=r"(w[i]) : "l"(p));
+        });
+    }
+    __device__ __forceinline__ void store(char *base, int64_t nface, int64_t face) const {
+        columns(base, nface, face, [&](char *p, int i, auto words) {
+#pragma unroll
+            for (int j = 0; j < decltype(words)::value; ++j) reinterpret_cast<uint32_t *>(p)[j] = w[i + j];
+        });
+    }
+};
 
 // ld16: plain 128-bit loads, for records that other threads of the same
 // kernel may have written before a barrier (sequential LocalAccTime1).
@@ -457,21 +515,11 @@ __device__ __forceinline__ bool riemann_flux(const Prim<R, DIM> r[2], const R nn
     return true;
 }
 
-// Interior face: reconstruction (REC 0 first order) and Riemann flux; one
-// gradient record's projections are formed before the other's, so one record
-// is dead before the next is read.
-template <typename R, int DIM, int FLUX, int REC, int LIM>
-__device__ __forceinline__ bool interior_flux(Prim<R, DIM> r[2], const GradRec<R, DIM> *gr0,
-                                              const GradRec<R, DIM> *gr1, const FaceRec<R, DIM> &fr,
-                                              const R nn[DIM], const Gas &gas, R flow[DIM + 2]) {
-    if (REC) {
-        R d0[DIM + 2], d1[DIM + 2];
-        project<R, DIM>(*gr0, fr.o0, d0);
-        project<R, DIM>(*gr1, REC == 1 ? fr.o0 : fr.o1, d1);
-        reconstruct<R, DIM, REC, LIM>(r, d0, d1, (R)gas.rm);
-    }
-    return riemann_flux<R, DIM, FLUX>(r, nn, gas, flow);
-}
+}  // namespace psst
+
+#include "lin_flux.cuh"
+
+namespace psst {
 
 // ---------------------------------------------------------------------------
 // face pass
@@ -486,38 +534,84 @@ __device__ __forceinline__ bool interior_flux(Prim<R, DIM> r[2], const GradRec<R
 //   reference adds the two sound speeds in the opposite order on the other
 //   side; IEEE addition is commutative) and S;
 //  LocalAccTime2 (:189-193): S |n_k|.
-// Register cap PSST_FACE_MAXNREG on the FP32 path (48: ten 128-thread blocks per SM;
-// PSST_FACE_MAXNREG_DM = 56 for the DM reconstruction, which spills at 48 and
-// measured 7% faster at 56).
+// Bound by the bytes it moves on large meshes (2.1M tets: 5.3 of 6.5 TB/s): hence
+// the packed columns (FaceCols) instead of whole face records. The blocks run
+// from the last face to the first: the cell pass before went forwards, so what it
+// wrote last is still in L2, and so is what this pass writes last when the next
+// cell pass starts with it (iteration of 440k tets in FP64 525 -> 514 us).
+// HLL and HLLC without DM in 3D or FP64 as straight-line code (lin_flux.cuh): face
+// pass 45.7 -> 43.4 us on 750k tets (FP32), 70.1 -> 64.9 on 440k (FP64). DM keeps the
+// branches, since most limiters of a flow leave by the first ones (113.8 -> 125.6
+// without), and so do AUSM (46.7 -> 48.3, 181k hexes, FP64) and 2D FP32 (25.4 -> 28.7).
 template <typename R, int DIM, int FLUX, int REC, int LIM, int LC>
-__global__ void __maxnreg__(PSST_BUDGET(R, REC == 1 ? PSST_FACE_MAXNREG_DM : PSST_FACE_MAXNREG, 128)) k_face(DevGrid g, DevState<R> st, DevWork<R> wk, Gas gas) {
+__global__ void __maxnreg__(PSST_BUDGET(R, REC == 1 ? PSST_FACE_MAXNREG_DM : DIM == 3 ? PSST_FACE_MAXNREG : 48, 128)) k_face(DevGrid g, DevState<R> st, DevWork<R> wk, Gas gas) {
     using FO = FaceOut<R, DIM>;
-    const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t f = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
     if (f >= g.nface) return;
     if (g.face_case && !g.case_active[g.face_case[f]]) return;  // stopped case (merged grids)
-    const FaceRec<R, DIM> fr = ldg(reinterpret_cast<const FaceRec<R, DIM> *>(g.frec) + f);
+    PackedFace<R, DIM, REC> fr;
+    fr.load(g.fcols, g.nface, f);
+    const int32_t c0 = (int32_t)fr.w[0], c1 = (int32_t)fr.w[1];
     R nn[DIM];
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) nn[k] = (R)fr.n[k];
-    const R S = (R)fr.S;
-    const Prim<R, DIM> p0 = unpack<R, DIM>(ldg(st.rec + fr.c0));
-    const Prim<R, DIM> p1 = unpack<R, DIM>(ldg(st.rec + fr.c1));
+    for (int k = 0; k < DIM; ++k) nn[k] = fr.value(1 + k);
+    const R S = fr.value(0);
+    const Prim<R, DIM> p0 = unpack<R, DIM>(ldg(st.rec + c0));
+    const Prim<R, DIM> p1 = unpack<R, DIM>(ldg(st.rec + c1));
     R flow[DIM + 2];
     if (f < g.nfi) {
         const GradRec<R, DIM> *grec = reinterpret_cast<const GradRec<R, DIM> *>(wk.grec);
         GradRec<R, DIM> g0, g1;
         if (REC) {
-            g0 = ldg(grec + fr.c0);
-            g1 = ldg(grec + fr.c1);
+            g0 = ldg(grec + c0);
+            g1 = ldg(grec + c1);
         }
         Prim<R, DIM> r[2] = {p0, p1};
-        if (!interior_flux<R, DIM, FLUX, REC, LIM>(r, &g0, &g1, fr, nn, gas, flow)) {
-            flag_error(wk.err, FLUX == 2 ? ERR_HLL : ERR_HLLC, f);
+        R d0[DIM + 2], d1[DIM + 2];
+        constexpr bool LIN = REC != 1 && FLUX != 1 && (DIM == 3 || sizeof(R) == 8);
+        bool fine = LIN;
+        if (REC) {
+            R off[DIM];
 #pragma unroll
-            for (int j = 0; j < DIM + 2; ++j) flow[j] = (R)0;
+            for (int k = 0; k < DIM; ++k) off[k] = fr.value(1 + DIM + k);
+            project<R, DIM>(g0, off, d0);
+            if (REC == 2)
+#pragma unroll
+                for (int k = 0; k < DIM; ++k) off[k] = fr.value(1 + (REC == 2 ? 2 * DIM : 0) + k);
+            project<R, DIM>(g1, off, d1);
+        }
+        if (LIN) {
+            if (REC) lin_reconstruct<R, DIM, REC, LIM>(r, d0, d1, (R)gas.rm, fine);
+            lin_flux<R, DIM, FLUX>(r, nn, gas, -1, flow, fine);
+        } else {
+            if (REC) reconstruct<R, DIM, REC, LIM>(r, d0, d1, (R)gas.rm);
+            if (!riemann_flux<R, DIM, FLUX>(r, nn, gas, flow)) {
+                flag_error(wk.err, FLUX == 2 ? ERR_HLL : ERR_HLLC, f);
+#pragma unroll
+                for (int j = 0; j < DIM + 2; ++j) flow[j] = (R)0;
+            }
+        }
+        if (LIN && !fine) {
+            PlainFace<R, DIM, REC, LIM> pf;
+            pf.r[0] = p0;
+            pf.r[1] = p1;
+            pf.flux = FLUX;
+            pf.edge = -1;
+            if (REC)
+#pragma unroll
+                for (int v = 0; v < DIM + 2; ++v) {
+                    pf.d0[v] = d0[v];
+                    pf.d1[v] = d1[v];
+                }
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) pf.n[k] = nn[k];
+            const bool ordered = PlainFace<R, DIM, REC, LIM>::run(&pf, &gas);
+            if (!ordered) flag_error(wk.err, FLUX == 2 ? ERR_HLL : ERR_HLLC, f);
+#pragma unroll
+            for (int j = 0; j < DIM + 2; ++j) flow[j] = ordered ? pf.flow[j] : (R)0;
         }
     } else {
-        boundary_flux<R, DIM>(fr.c0 >= g.nint ? p0 : p1, nn, gas, flow);
+        boundary_flux<R, DIM>(c0 >= g.nint ? p0 : p1, nn, gas, flow);
     }
     FO o;
 #pragma unroll
@@ -548,6 +642,25 @@ __global__ void __maxnreg__(PSST_BUDGET(R, REC == 1 ? PSST_FACE_MAXNREG_DM : PSS
         for (int k = 0; k < DIM; ++k) o.v[FO::Q0 + k] = S * fabs(nn[k]);
     }
     st16(reinterpret_cast<FO *>(wk.fout) + f, o);
+}
+
+// The face pass's columns (FaceCols) from the face records.
+template <typename R, int DIM, int REC>
+__global__ void __launch_bounds__(256) k_face_columns(DevGrid g, char *cols) {
+    const int32_t f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= g.nface) return;
+    const FaceRec<R, DIM> fr = ldg(reinterpret_cast<const FaceRec<R, DIM> *>(g.frec) + f);
+    PackedFace<R, DIM, REC> o;
+    o.w[0] = (uint32_t)fr.c0;
+    o.w[1] = (uint32_t)fr.c1;
+    o.put(0, (R)fr.S);
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+        o.put(1 + k, (R)fr.n[k]);
+        if constexpr (REC >= 1) o.put(1 + DIM + k, fr.o0[k]);
+        if constexpr (REC == 2) o.put(1 + 2 * DIM + k, fr.o1[k]);
+    }
+    o.store(cols, g.nface, f);
 }
 
 // ---------------------------------------------------------------------------
@@ -910,7 +1023,7 @@ __device__ __forceinline__ void gradient_cell(const DevGrid &g, const CellRec<R>
 }
 
 template <typename R, int DIM, int GRAD, int CELLLIM>
-__global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_GRAD_MINB, 1)) k_gradient(DevGrid g, DevState<R> st, DevWork<R> wk) {
+__global__ void __launch_bounds__(256, PSST_BUDGET(R, DIM == 3 ? PSST_GRAD_MINB : 3, 1)) k_gradient(DevGrid g, DevState<R> st, DevWork<R> wk) {
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= g.nint) return;
     if (g.cell_case && !g.case_active[g.cell_case[c]]) return;  // stopped case
@@ -994,26 +1107,56 @@ __device__ __forceinline__ RkIn<NV> rk_load(const DevGrid &g, const DevWork<R> &
 // RK stage update of one cell given its residual (psstFiniteVolumeGrid.cpp:324-346):
 // w = prev_w - dt*a*res/V in FP64, primitives, norms; returns the new record.
 // w and dt are stored only when `keep` is set: inside a whole iteration only
-// the last stage's values are ever read (the next iteration's first stage
-// loads w; stages 2.. load the stage-start copy pw).
+// the last stage's values are ever read, and until then w keeps the iteration's
+// start, which every stage loads. (The stage-by-stage API stores w after every
+// stage and the start in pw: `save`, on its first stage.)
 template <typename R, int DIM>
 __device__ __forceinline__ CellRec<R> rk_update(const DevGrid &g, const DevWork<R> &wk, const Gas &gas,
-                                                const RkIn<DIM + 2> &in, double dt, double alpha, int first_stage,
+                                                const RkIn<DIM + 2> &in, double dt, double alpha, bool save,
                                                 bool keep, int32_t c, const R res[DIM + 2], double sq[DIM + 2],
                                                 double mx[DIM + 2]) {
     constexpr int NV = DIM + 2;
     // FP64 (parity) path: the reference's operation order, one division per
-    // component; FP32 path: one reciprocal per cell (its own rounding)
+    // component; FP32 path: one reciprocal per cell (its own rounding). As
+    // straight-line divisions with the bits of `/`, or by `/` itself where an
+    // operand is out of their range.
     constexpr bool EXACT = sizeof(R) == 8;
-    const double vol = in.vol;
-    const double step = EXACT ? 0.0 : dt * alpha / vol;
-    double w[NV];
+    double w[NV], rho, T;
+    R u[DIM];
+    auto update = [&](auto plain) {
+        constexpr bool P = decltype(plain)::value;
+        auto recip = [](double d) { return P ? 1.0 / d : lin_recip(d); };
+        auto over = [](double x, double d, double y) { return P ? x / d : lin_quot(x, d, y); };
+        const double rvol = EXACT && P ? 0.0 : recip(in.vol);
+        const double step = EXACT ? 0.0 : over(dt * alpha, in.vol, rvol);
+        bool fine = den_ok(in.vol) && den_ok(gas.cv);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double x = EXACT ? dt * alpha * (double)res[v] : dt * alpha;
+            w[v] = EXACT ? in.pw[v] - over(x, in.vol, rvol) : in.pw[v] - step * (double)res[v];
+            fine = fine && zero_or_in_range(x) && zero_or_in_range(w[v]);
+        }
+        rho = w[DIM];
+        fine = fine && den_ok(rho);
+        const double irho = EXACT && P ? 0.0 : recip(rho);
+        double vs = 0.0;
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) {
+            const double uk = EXACT ? over(w[k], rho, irho) : w[k] * irho;
+            u[k] = (R)uk;
+            vs += uk * uk;
+        }
+        const double e = (EXACT ? over(w[DIM + 1], rho, irho) : w[DIM + 1] * irho) - (vs * 0.5);
+        fine = fine && zero_or_in_range(e);
+        const double rcv = recip(gas.cv);
+        T = EXACT ? over(e, gas.cv, rcv) : e * rcv;
+        return fine;
+    };
+    if (!update(std::false_type())) update(std::true_type());
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         const int64_t idx = (int64_t)v * g.nint + c;
-        const double pw = in.pw[v];
-        if (first_stage) wk.pw[idx] = pw;
-        w[v] = EXACT ? pw - dt * alpha * (double)res[v] / vol : pw - step * (double)res[v];
+        if (save) wk.pw[idx] = in.pw[v];
         if (keep) wk.w[idx] = w[v];
         const double rv = (double)res[v];
         const double ar = fabs(rv);
@@ -1021,18 +1164,6 @@ __device__ __forceinline__ CellRec<R> rk_update(const DevGrid &g, const DevWork<
         sq[v] += rv * rv;
         if (!(rv - rv == 0.0)) flag_error(wk.err, ERR_NONFINITE_RES, c);
     }
-    const double rho = w[DIM];
-    const double irho = EXACT ? 0.0 : 1.0 / rho;
-    double vs = 0.0;
-    R u[DIM];
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) {
-        const double uk = EXACT ? w[k] / rho : w[k] * irho;
-        u[k] = (R)uk;
-        vs += uk * uk;
-    }
-    const double T = EXACT ? ((w[DIM + 1] / rho) - (vs * 0.5)) / gas.cv
-                           : ((w[DIM + 1] * irho) - (vs * 0.5)) * (1.0 / gas.cv);
     const double p = rho * gas.rm * T;
     if (!(rho > 0.0 && T > 0.0)) flag_error(wk.err, ERR_BAD_STATE, c);
     if (keep) wk.dt[c] = dt;
@@ -1178,7 +1309,7 @@ __global__ void __launch_bounds__(256) k_norm_finish(const double *part, int nbl
 // contiguous in device order) reduce first; cs < 0 contributes nothing. NaN
 // never enters (mx skips it, as the reference's `if (res < |r|)` does).
 // Called by all 32 lanes of every warp.
-template <int NV>
+template <int NV, bool FMAX>
 __device__ __forceinline__ void case_max(unsigned long long *cl, int32_t cs, const double mx[NV]) {
     const int32_t c0 = __shfl_sync(FULL, cs, 0);
     if (__all_sync(FULL, cs == c0)) {
@@ -1187,7 +1318,8 @@ __device__ __forceinline__ void case_max(unsigned long long *cl, int32_t cs, con
         for (int v = 0; v < NV; ++v) {
             double m = mx[v];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(FULL, m, o));
+            for (int o = FMAX ? 0 : 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(FULL, m, o));
+            if (FMAX) m = (double)__uint_as_float(__reduce_max_sync(FULL, __float_as_uint((float)m)));
             if ((threadIdx.x & 31) == 0 && m > 0.0)
                 atomicMax(cl + (int64_t)c0 * NV + v, (unsigned long long)__double_as_longlong(m));
         }
@@ -1256,29 +1388,53 @@ __global__ void __launch_bounds__(256) k_loop_control(CaseStop cs, int32_t ncase
 // reduces its lanes (shuffle trees) into a shared slot, and the last warp of
 // the block to arrive sums the slots in warp order and writes out[2 NV] (sum
 // res^2, max |res|); the other warps leave at once. `count` must be zero at
-// the block's start. FMAX: the maxima are FP32 values, reduced as floats.
+// the block's start. FMAX: the maxima are FP32 values, reduced as integers (their
+// bits, non-negative floats). A warp's sums are scattered while they are formed --
+// each step hands half of a lane's components to its partner -- in 8 shuffles of a
+// double for 5 components instead of 25.
+template <int NV, class Op>
+__device__ __forceinline__ void scatter_reduce(const double s[NV], double *red, Op op) {
+    static_assert(NV == 4 || NV == 5, "components");
+    constexpr int H = (NV + 1) / 2;  // kept by the lower half-warp; the upper keeps NV - H
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    auto both = [&](double keep, double give, int o) { return op(keep, __shfl_xor_sync(FULL, give, o)); };
+    double t[3] = {};
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const double hi = H + i < NV ? s[H + i] : 0.0;
+        t[i] = both(b4 ? hi : s[i], b4 ? s[i] : hi, 16);
+    }
+    double x;
+    int comp = b4 ? H : 0;
+    if (NV == 4) {
+        x = both(b3 ? t[1] : t[0], b3 ? t[0] : t[1], 8);
+        x = both(x, x, 4);
+        comp += b3;
+    } else {  // components (0, 1) and 2 of the half
+        const double a = both(b3 ? t[2] : t[0], b3 ? t[0] : t[2], 8), b = both(t[1], t[1], 8);
+        x = both(b3 ? a : b2 ? b : a, b3 ? a : b2 ? a : b, 4);
+        comp += b3 ? 2 : b2;
+    }
+    x = both(x, x, 2);
+    x = both(x, x, 1);
+    if ((lane & 3) == 0 && comp < NV && (NV == 4 ? !b2 : !(b3 && b2))) red[comp * 32 + (threadIdx.x >> 5)] = x;
+}
 template <int NV, bool FMAX = false>
 __device__ __forceinline__ void lastwarp_partials(double sq[NV], double mx[NV], double *out, unsigned *count) {
     __shared__ double red[2 * NV][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    scatter_reduce<NV>(sq, &red[0][0], [](double a, double b) { return a + b; });
+    if (FMAX) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        double x = sq[v], m = mx[v];
-        float mf = (float)m;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            x += __shfl_down_sync(FULL, x, o);
-            if (FMAX)
-                mf = fmaxf(mf, __shfl_down_sync(FULL, mf, o));
-            else
-                m = fmax(m, __shfl_down_sync(FULL, m, o));
+        for (int v = 0; v < NV; ++v) {
+            const unsigned m = __reduce_max_sync(FULL, __float_as_uint((float)mx[v]));
+            if (lane == 0) red[NV + v][wid] = (double)__uint_as_float(m);
         }
-        if (FMAX) m = (double)mf;
-        if (lane == 0) {
-            red[v][wid] = x;
-            red[NV + v][wid] = m;
-        }
+    } else {
+        scatter_reduce<NV>(mx, &red[NV][0], [](double a, double b) { return fmax(a, b); });
     }
+    __syncwarp();
     unsigned last = 0;
     if (lane == 0) {
         __threadfence_block();
@@ -1392,6 +1548,9 @@ __device__ __forceinline__ void gather_residual(const DevGrid &g, const FaceOut<
 // ghost cells, and the block's norm partials for this stage (formed by the
 // block's last warp to finish, so no warp waits at a block barrier;
 // k_norm_reduce turns the stages' partials into the iteration's columns).
+// (Two shuffle reductions of five values used to take 25 double shuffles each, and
+// the start-of-iteration state a copy: 93.0 -> 83.9 us on 2.1M tets without them and
+// with the cells' face orders read only where they differ.)
 // At least 4 blocks of 256 per SM (64 registers): the pass is bound by the
 // latency of its gathers, and the occupancy gained outweighs a 24-byte spill
 // (0.61 -> 0.56 ms per launch on 6M tets, FP32).
@@ -1419,9 +1578,8 @@ template <typename R, int DIM, int LC, bool BATCH>
 __global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_CELL_MINB, 2)) k_cell(DevGrid g, DevState<R> cur, DevState<R> nxt, DevWork<R> wk, Gas gas,
                                               double cfl, double dt_uniform, double alpha, int stage,
                                               int kstage, int it_slot) {
-    // stage: bit 0 first stage of the iteration, bit 1 last stage; kstage: its index
+    // stage: bit 1 last stage of the iteration; kstage: its index
     using FO = FaceOut<R, DIM>;
-    const int first_stage = stage & 1;
     constexpr int NV = DIM + 2;
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     __shared__ unsigned warps_done;  // lastwarp_partials
@@ -1439,13 +1597,14 @@ __global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_CELL_MINB, 2)) k_cell
     if (run) {
         const FO *fo = reinterpret_cast<const FO *>(wk.fout);
         const R *csr_s = reinterpret_cast<const R *>(g.csr_s);
-        const RkIn<NV> rin = rk_load<R, NV>(g, wk, first_stage, c);
+        const RkIn<NV> rin = rk_load<R, NV>(g, wk, true, c);  // w keeps the iteration's start until its last stage
         const int32_t b = g.kuni ? c * g.kuni : g.csr_ptr[c], K = g.kuni ? g.kuni : g.csr_ptr[c + 1] - b;
-        const uint64_t perm = g.wperm[c];
         // When the cell's own face order is the face-loop order (the usual
         // case: faces are wired zone by zone in file order, and files list
         // zones in ascending id), residual and time step share one pass.
-        const bool one_pass = LC != 0 && perm == (0xFEDCBA9876543210ull & ((K >= 16) ? ~0ull : ((1ull << (4 * K)) - 1)));
+        const uint64_t straight = 0xFEDCBA9876543210ull & ((K >= 16) ? ~0ull : ((1ull << (4 * K)) - 1));
+        const uint64_t perm = g.same_order ? straight : g.wperm[c];
+        const bool one_pass = LC != 0 && perm == straight;
         R res[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) res[v] = (R)0;
@@ -1523,7 +1682,7 @@ __global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_CELL_MINB, 2)) k_cell
             }
             dt = (double)((R)cfl * (R)g.V[c] / den);
         }
-        const CellRec<R> nrec = rk_update<R, DIM>(g, wk, gas, rin, dt, alpha, first_stage, (stage & 2) != 0, c, res,
+        const CellRec<R> nrec = rk_update<R, DIM>(g, wk, gas, rin, dt, alpha, false, (stage & 2) != 0, c, res,
                                                   sq, mx);
         st16(nxt.rec + c, nrec);
         const int32_t g0 = g.gptr[c], g1 = g.gptr[c + 1];
@@ -1535,7 +1694,7 @@ __global__ void __launch_bounds__(256, PSST_BUDGET(R, PSST_CELL_MINB, 2)) k_cell
             }
         }
     }
-    if (BATCH) case_max<NV>(wk.case_linf + (int64_t)it_slot * g.ncase * NV, run ? g.cell_case[c] : -1, mx);
+    if (BATCH) case_max<NV, sizeof(R) == 4>(wk.case_linf + (int64_t)it_slot * g.ncase * NV, run ? g.cell_case[c] : -1, mx);
     lastwarp_partials<NV, sizeof(R) == 4>(sq, mx, wk.l2part + ((int64_t)kstage * gridDim.x + blockIdx.x) * 2 * NV,
                                           &warps_done);
 }
@@ -1563,7 +1722,7 @@ __device__ __forceinline__ void update_from_buffers(const DevGrid &g, const DevS
         dt = local_time<R, DIM, 1, true>(g, cur.rec, nxt.rec, gas, cfl, dt_uniform, c, own);
     else
         dt = local_time<R, DIM, LC, false>(g, cur.rec, nxt.rec, gas, cfl, dt_uniform, c, own);
-    st16(nxt.rec + c, rk_update<R, DIM>(g, wk, gas, rin, dt, alpha, first_stage, true, c, res, sq, mx));
+    st16(nxt.rec + c, rk_update<R, DIM>(g, wk, gas, rin, dt, alpha, first_stage != 0, true, c, res, sq, mx));
 }
 
 template <typename R, int DIM, int LC, bool GATHER>

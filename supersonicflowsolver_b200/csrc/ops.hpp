@@ -87,6 +87,9 @@ struct Ops {
     // the static face data of its items (FaceData), from the grid's arrays: mate
     // per CSR entry the same face's entry in the cell across, pos per cell its
     // place item * 32 + slot
+    // the face pass's columns: their size (FaceCols), and filling them from the face records
+    static size_t face_columns_bytes(int dim, int rec, int64_t nface);
+    static void face_columns(int dim, int rec, const DevGrid &g, char *cols, cudaStream_t s);
     static void resident_build(int dim, int rec, int grad, const DevGrid &g, const int32_t *cells32,
                                const uint32_t *lowmask, const int32_t *mate, const int32_t *pos, int nitems,
                                int rounds, void *faces, void *cells, cudaStream_t s);

@@ -149,6 +149,33 @@ void Ops<R>::face(int dim, int flux, int rec, int lim, int lc, const DevGrid &g,
         face_f<R, 3>(flux, rec, lim, lc, g, st, wk, gas, s);
 }
 
+template <typename R, int DIM>
+static size_t face_columns_bytes_d(int rec, int64_t n) {
+    return (size_t)(rec == 0 ? FaceCols<R, DIM, 0>::bytes(n) : rec == 1 ? FaceCols<R, DIM, 1>::bytes(n) : FaceCols<R, DIM, 2>::bytes(n));
+}
+template <typename R>
+size_t Ops<R>::face_columns_bytes(int dim, int rec, int64_t nface) {
+    return dim == 2 ? face_columns_bytes_d<R, 2>(rec, nface) : face_columns_bytes_d<R, 3>(rec, nface);
+}
+template <typename R, int DIM>
+static void face_columns_d(int rec, const DevGrid &g, char *cols, cudaStream_t s) {
+    const int nb = nblocks(g.nface, 256);
+    if (rec == 0)
+        k_face_columns<R, DIM, 0><<<nb, 256, 0, s>>>(g, cols);
+    else if (rec == 1)
+        k_face_columns<R, DIM, 1><<<nb, 256, 0, s>>>(g, cols);
+    else
+        k_face_columns<R, DIM, 2><<<nb, 256, 0, s>>>(g, cols);
+}
+template <typename R>
+void Ops<R>::face_columns(int dim, int rec, const DevGrid &g, char *cols, cudaStream_t s) {
+    if (g.nface == 0) return;
+    if (dim == 2)
+        face_columns_d<R, 2>(rec, g, cols, s);
+    else
+        face_columns_d<R, 3>(rec, g, cols, s);
+}
+
 // ---- cell pass (parallel modes) ----
 template <typename R, int DIM>
 static void cell_d(int lc, const DevGrid &g, const DevState<R> &cur, const DevState<R> &nxt, const DevWork<R> &wk,

@@ -81,6 +81,7 @@ struct Layout {
     std::vector<int32_t> res_cells32, res_item_level;
     std::vector<uint32_t> res_lowmask;
     std::vector<uint64_t> wperm;
+    bool same_order = false;  // every wperm is the identity
     std::vector<double> S, n, xf, beta, V, xc, lsq_r, vk_eps2, z_u, z_p, z_T;
 };
 
@@ -270,6 +271,11 @@ void build_layout(const psst_grid &G, const psst_scheme &sc, Layout &L) {
             L.wperm[d] = perm;
         }
     });
+    L.same_order = true;
+    for (int32_t d = 0; d < L.nint && L.same_order; ++d) {
+        const int k = L.csr_ptr[d + 1] - L.csr_ptr[d];
+        L.same_order = L.wperm[d] == (0xFEDCBA9876543210ull & (k >= 16 ? ~0ull : (1ull << (4 * k)) - 1));
+    }
     // ghost tables and boundary zones; ghosts are sorted by interior neighbour,
     // so each interior cell owns a contiguous ghost range [gptr[d], gptr[d+1])
     L.g_nb.resize(L.nghost);
@@ -579,8 +585,15 @@ struct psst_solver {
         if (hnorm) cudaFreeHost(hnorm);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
+        if (ev_cell) cudaEventDestroy(ev_cell);
+        if (ev_norm) cudaEventDestroy(ev_norm);
+        if (norm_stream) cudaStreamDestroy(norm_stream);
         if (own_stream) cudaStreamDestroy(own_stream);
     }
+    // Residual columns on a stream of their own (see NormFork).
+    cudaStream_t norm_stream = nullptr;
+    cudaEvent_t ev_cell = nullptr, ev_norm = nullptr;
+    bool norm_fork = false, norm_pending = false;
 };
 
 namespace {
@@ -614,6 +627,11 @@ void alloc_state(psst_solver *s, const psst_grid &G) {
         s->g.frec = s->upload(build_face_records<R, 2>(G, s->L, s->rec));
     else
         s->g.frec = s->upload(build_face_records<R, 3>(G, s->L, s->rec));
+    char *cols = (char *)s->dalloc_bytes(Ops<R>::face_columns_bytes(dim, s->rec, nface));
+    s->g.fcols = cols;
+    ck(cudaStreamSynchronize(nullptr), "upload");  // the records are on the device
+    Ops<R>::face_columns(dim, s->rec, s->g, cols, s->stream);
+    ck(cudaStreamSynchronize(s->stream), "face columns");
     {  // face area per CSR entry, rounded to R as the face pass rounds it
         std::vector<R> cs(s->L.csr_ent.size());
         for (size_t q = 0; q < cs.size(); ++q) cs[q] = (R)s->L.S[s->L.csr_ent[q] >> 1];
@@ -714,6 +732,30 @@ void check_err(psst_solver *s, const int32_t *err_dev) {
 
 enum Kind { K_GRADIENT = 0, K_FACE = 1, K_CELL = 2, K_GHOST = 3, K_NORM = 4 };
 
+// While alive, each iteration's norm reduction (13 us of latency: small blocks, two
+// levels) runs beside the next iteration's gradient and first face pass, which
+// need nothing of it, instead of before them: 4 to 5% of an iteration of 750k
+// tets (FP32) or 181k hexes (FP64). In a graph the fork costs nothing; without
+// one it is four more host calls an iteration, so only where the device has
+// enough to do (65536 cells: an iteration takes some 100 us).
+struct NormFork {
+    psst_solver *s;
+    explicit NormFork(psst_solver *s_, bool captured) : s(s_) {
+        if (!captured && s->L.nint < 65536) return;
+        if (!s->norm_stream) {
+            ck(cudaStreamCreateWithFlags(&s->norm_stream, cudaStreamNonBlocking), "stream");
+            ck(cudaEventCreateWithFlags(&s->ev_cell, cudaEventDisableTiming), "event");
+            ck(cudaEventCreateWithFlags(&s->ev_norm, cudaEventDisableTiming), "event");
+        }
+        s->norm_fork = true;
+    }
+    ~NormFork() { s->norm_fork = false; }
+};
+void join_norms(psst_solver *s) {
+    if (s->norm_pending) ck(cudaStreamWaitEvent(s->stream, s->ev_norm, 0), "stream wait");
+    s->norm_pending = false;
+}
+
 // One RK stage. The parallel modes run face pass -> cell pass (the cell pass
 // also updates ghosts and finishes the norms); the sequential LocalAccTime1
 // mode and the stage-by-stage API (gather == false: residual already in
@@ -730,12 +772,21 @@ void one_stage(psst_solver *s, int k, int it_slot, bool gather, Mark &&mark) {
         mark(K_FACE);
     }
     if (gather && !s->seq) {
-        const int stage = (k == 0 ? 1 : 0) | (k == s->sc.rk_level - 1 ? 2 : 0);
+        const int stage = k == s->sc.rk_level - 1 ? 2 : 0;
+        if (k == 0) join_norms(s);  // the cell pass writes the partials that the norm kernel reads
         Ops<R>::cell(s->dim, s->sc.lc, s->g, cur, nxt, w, s->gas, s->sc.cfl, s->dt_uniform, s->sc.rk[k], stage, k,
                      it_slot, s->stream);
         mark(K_CELL);
         if (k == s->sc.rk_level - 1) {  // the iteration's residual columns
-            Ops<R>::norm_reduce(s->dim, s->g, w, s->sc.rk_level, it_slot, s->stream);
+            if (s->norm_fork) {
+                ck(cudaEventRecord(s->ev_cell, s->stream), "event");
+                ck(cudaStreamWaitEvent(s->norm_stream, s->ev_cell, 0), "stream wait");
+                Ops<R>::norm_reduce(s->dim, s->g, w, s->sc.rk_level, it_slot, s->norm_stream);
+                ck(cudaEventRecord(s->ev_norm, s->norm_stream), "event");
+                s->norm_pending = true;
+            } else {
+                Ops<R>::norm_reduce(s->dim, s->g, w, s->sc.rk_level, it_slot, s->stream);
+            }
             mark(K_NORM);
         }
     } else {
@@ -788,11 +839,7 @@ void build_resident(psst_solver *s) {
     s->res_blocks = std::min(nitems, maxb);
     w.period = L.res_period;
     w.seq = s->seq;
-    w.same_order = true;
-    for (int32_t d = 0; d < L.nint && w.same_order; ++d) {
-        const int kd = L.csr_ptr[d + 1] - L.csr_ptr[d];
-        w.same_order = L.wperm[d] == (0xFEDCBA9876543210ull & (kd >= 16 ? ~0ull : (1ull << (4 * kd)) - 1));
-    }
+    w.same_order = s->g.same_order != 0;
     w.nitems = nitems;
     w.smem_items = items;
     std::vector<int32_t> ptr(1, 0);
@@ -944,6 +991,7 @@ void iterations(psst_solver *s, int n_iter, Mark &&mark) {
         resident_run<R>(s, n_iter, mark);
         return;
     }
+    s->norm_pending = false;
     for (int it = 0; it < n_iter; ++it) {
         if (s->sc.order == 2) {
             Ops<R>::gradient(s->dim, s->sc.grad, s->celllim, s->g, states<R>(s)[s->cur], w, s->stream);
@@ -955,6 +1003,7 @@ void iterations(psst_solver *s, int n_iter, Mark &&mark) {
             mark(K_NORM);
         }
     }
+    join_norms(s);
 }
 
 // n_iter iterations. With graphs on, the whole call (norm reset + every
@@ -969,6 +1018,7 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
     if (resident_active(s) && resident_run<R>(s, n_iter, count)) {
         // one launch, which wrote every residual column
     } else if (s->use_graphs) {
+        const NormFork fork(s, true);
         const std::pair<int, int> key(n_iter, s->cur);
         auto it = s->graphs.find(key);
         if (it == s->graphs.end()) {
@@ -995,6 +1045,7 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
         }
         ck(cudaGraphLaunch(it->second, s->stream), "graph launch");
     } else {
+        const NormFork fork(s, false);
         zero_norms<R>(s, n_iter);
         iterations<R>(s, n_iter, count);
     }
@@ -1065,7 +1116,7 @@ int64_t run_to_stop(psst_solver *s, int64_t max_iter, int chunk, double *res_lin
         cudaGraph_t gr = nullptr;
         ck(cudaGraphCreate(&gr, 0), "graph");
         int64_t launches = 0;
-        try {
+        try {  // without NormFork: parallel branches in a loop body cost more than they hide (batch of 48: 26 -> 36 ms)
             cudaGraphConditionalHandle h;
             ck(cudaGraphConditionalHandleCreate(&h, gr, 1, cudaGraphCondAssignDefault), "graph condition");
             cudaGraphNodeParams p{};
@@ -1499,6 +1550,7 @@ extern "C" psst_status psst_solver_create(const psst_grid *G, const psst_scheme 
     g.csr_ent = s->upload(L.csr_ent);
     g.csr_nb = s->upload(L.csr_nb);
     g.wperm = s->upload(L.wperm);
+    g.same_order = L.same_order;
     g.lsq_r = s->upload(L.lsq_r);
     g.vk_eps2 = s->upload(L.vk_eps2);
     g.rank = s->upload(L.rank);

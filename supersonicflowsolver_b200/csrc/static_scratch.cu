@@ -84,9 +84,7 @@ __global__ void __launch_bounds__(256) k_static_face(int32_t nint, int32_t nall,
         boundary_flux<double, DIM>(soa_prim<DIM>(prim, nall, a >= nint ? a : b), nn, gas, flow);
     } else {
         Prim<double, DIM> r[2] = {soa_prim<DIM>(prim, nall, a), soa_prim<DIM>(prim, nall, b)};
-        FaceRec<double, DIM> unused{};
-        GradRec<double, DIM> g0, g1;
-        if (!interior_flux<double, DIM, FLUX, 0, 1>(r, &g0, &g1, unused, nn, gas, flow)) {
+        if (!riemann_flux<double, DIM, FLUX>(r, nn, gas, flow)) {
             int32_t *err = reinterpret_cast<int32_t *>(fs + 5 * kMaxFaces);
             flag_error(err, FLUX == 2 ? ERR_HLL : ERR_HLLC, f);
 #pragma unroll
