@@ -858,11 +858,13 @@ extern "C" psst_status psst_mlp_create(int device, uint64_t seed, psst_mlp **out
     m->wbf = dmalloc<bf16>(m->allocs, m->net.nwbf);
     m->status = dmalloc<int>(m->allocs, 2);
     for (int l = 0; l < kHidden; ++l) m->maps.w[l] = box_map(m->wbf + m->net.offWbf[l], kWidth, net_din(l));
-    ck(cudaMemcpy(m->p, h.data(), off * sizeof(float), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemset(m->m1, 0, off * sizeof(float)), "memset");
-    ck(cudaMemset(m->m2, 0, off * sizeof(float)), "memset");
-    ck(cudaMemset(m->g, 0, off * sizeof(float)), "memset");
-    ck(cudaMemset(m->status, 0, 2 * sizeof(int)), "memset");
+    // on the stream of the kernel that reads them: a copy from pageable memory on the
+    // default stream may still be on its way when the call returns
+    ck(cudaMemcpyAsync(m->p, h.data(), off * sizeof(float), cudaMemcpyHostToDevice, m->stream), "upload");
+    ck(cudaMemsetAsync(m->m1, 0, off * sizeof(float), m->stream), "memset");
+    ck(cudaMemsetAsync(m->m2, 0, off * sizeof(float), m->stream), "memset");
+    ck(cudaMemsetAsync(m->g, 0, off * sizeof(float), m->stream), "memset");
+    ck(cudaMemsetAsync(m->status, 0, 2 * sizeof(int), m->stream), "memset");
     k_to_bf16<<<nb(off / 4), 256, 0, m->stream>>>(m->p, m->net, m->wbf);
     ck(cudaStreamSynchronize(m->stream), "init");
     *out = m.release();
@@ -886,10 +888,10 @@ extern "C" psst_status psst_mlp_set_params(psst_mlp *m, const float *in, int64_t
     ck(cudaSetDevice(m->device), "cudaSetDevice");
     ck(cudaMemcpyAsync(m->p, in, n * sizeof(float), cudaMemcpyHostToDevice, m->stream), "copy");
     k_to_bf16<<<nb(n / 4), 256, 0, m->stream>>>(m->p, m->net, m->wbf);
+    ck(cudaMemsetAsync(m->m1, 0, n * sizeof(float), m->stream), "memset");
+    ck(cudaMemsetAsync(m->m2, 0, n * sizeof(float), m->stream), "memset");
     ck(cudaStreamSynchronize(m->stream), "sync");
     m->step = 0;
-    ck(cudaMemset(m->m1, 0, n * sizeof(float)), "memset");
-    ck(cudaMemset(m->m2, 0, n * sizeof(float)), "memset");
     MLP_END
 }
 

@@ -900,6 +900,7 @@ void build_resident(psst_solver *s) {
         s->res_proj_bytes = bytes.proj;
         s->res_proj = base + o_proj;
     }
+    ck(cudaStreamSynchronize(nullptr), "upload");  // the grid's tables are on the device
     Ops<R>::resident_build(s->dim, s->rec, s->sc.order == 2 ? s->sc.grad : 0, s->g, w.cells32,
                            L.res_lowmask.empty() ? nullptr : (const uint32_t *)(base + o_low),
                            (const int32_t *)(base + o_mate), (const int32_t *)(base + o_pos), nitems, w.rounds,
