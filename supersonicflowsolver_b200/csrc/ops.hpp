@@ -15,7 +15,7 @@ constexpr int kWfBlock = 128;  // threads per CTA of k_resident
 constexpr int kWfLanes = 4;    // lanes per cell in k_resident (cells per work item: 32)
 
 constexpr int kWfSyncWords = 96;  // k_resident's counter and flag words (three 128-byte lines)
-constexpr int kNormReduceBlocks = 296;  // blocks of k_norm_reduce (first level of its two-level sum): two per SM
+constexpr int kNormReduceBlocks = 296;  // most blocks a stage of k_norm_reduce (first level of its two-level sum)
 inline int nblocks(int64_t n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
 template <typename R>

@@ -213,7 +213,9 @@ template <typename R>
 void Ops<R>::norm_reduce(int dim, const DevGrid &g, const DevWork<R> &wk, int nstage, int it_slot, cudaStream_t s) {
     if (g.nint == 0) return;
     const int nblk = nblocks(g.nint, g.blk_cell);
-    const dim3 grid((unsigned)std::min(nblk, kNormReduceBlocks), (unsigned)nstage);
+    // some 128 partials a block: more blocks make the second level and the count of finished ones
+    // the longer part (18.5 us with 296 whatever the mesh, 12.5 with 30 to 90)
+    const dim3 grid((unsigned)std::max(std::min(nblk / 128, kNormReduceBlocks), 1), (unsigned)nstage);
     if (dim == 2)
         k_norm_reduce<4><<<grid, 64 * 4, 0, s>>>(wk.l2part, nblk, nstage, g.nint, wk.l2mid, wk.ticket, wk.linf, wk.l2,
                                                  it_slot);
