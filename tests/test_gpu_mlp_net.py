@@ -74,3 +74,46 @@ def test_train_step_is_adam_on_the_gradients():
         # float32 0.9 and 0.999 differ from the decimal ones by 2^-24 and 2^-24 / 0.001 relative to 1 - b:
         # 2.4e-7 and 2e-5 in the two corrections, which cancel against those of m and v only in part
         assert np.abs(net.params() - want).max() <= 2e-5 * 1.1 * lr + 2.0 ** -24
+
+
+HARNESS = r"""
+#include <cuda_runtime.h>
+#include "exact.cuh"
+__global__ void k(const float *a, const float *b, float *q, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) q[i] = psst::rn_div(a[i], b[i]);
+}
+extern "C" int run(const float *a, const float *b, float *q, int n) {
+    float *d[3];
+    for (int i = 0; i < 3; ++i)
+        if (cudaMalloc(&d[i], n * 4)) return 1;
+    cudaMemcpy(d[0], a, n * 4, cudaMemcpyHostToDevice);
+    cudaMemcpy(d[1], b, n * 4, cudaMemcpyHostToDevice);
+    k<<<(n + 255) / 256, 256>>>(d[0], d[1], d[2], n);
+    const int e = cudaMemcpy(q, d[2], n * 4, cudaMemcpyDeviceToHost);
+    for (int i = 0; i < 3; ++i) cudaFree(d[i]);
+    return e;
+}
+"""
+
+
+def test_silu_quotients_have_the_bits_of_the_division(tmp_path):
+    """z / (1 + e^-z) and 1 / (1 + e^-z) over the range that takes the straight-line quotient."""
+    import ctypes
+    import os
+    import subprocess
+
+    src, lib = tmp_path / "h.cu", str(tmp_path / "h.so")
+    src.write_text(HARNESS)
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "supersonicflowsolver_b200", "csrc")
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-I", csrc, "-shared",
+                    "-Xcompiler", "-fPIC", str(src), "-o", lib], check=True)
+    L = ctypes.CDLL(lib)
+    rng = np.random.default_rng(0)
+    n = 1 << 22
+    z = np.concatenate([rng.uniform(-87, 87, n), rng.normal(0, 2, n)]).astype(np.float32)
+    b = (np.float32(1) + np.exp(-z)).astype(np.float32)
+    for a in (z, np.ones_like(z)):
+        q = np.empty_like(z)
+        assert L.run(*(v.ctypes.data_as(ctypes.c_void_p) for v in (a, b, q)), len(z)) == 0
+        assert np.array_equal(q, a / b)
