@@ -179,18 +179,17 @@ def traffic_model(grid, nnz, kind, precision=32):
     nint, ngh, nf = grid.ninterior, grid.nghost, grid.nface
     K = nnz / nint
     if kind == "face":
-        # per face: face record read (64: c0,c1 (2i), S (g), n (3g), two FP32 offset vectors)
+        # per face: packed columns read (48: c0,c1 (2i), and S, n (3), two offset vectors in FP32)
         # and the face output record written (32: flux*area 5s, time-step terms 3s);
         # per interior cell: state record (32) + limited-gradient record (64); ghosts: state (32)
-        return nf * (64 + 32) + nint * (32 + 64) + ngh * 32
+        return nf * (48 + 32) + nint * (32 + 64) + ngh * 32
     if kind == "cell":
-        # per cell: CSR ptr (i) + K entries (i) + K face areas (s) + own-order perm (8) + V (g) +
-        # the stage-start FP64 state read (5x8) + new state record (32) + ghost ptr (i), and,
-        # averaged over the S stages of an iteration, the stage-start copy written on the first
-        # stage and w and dt written on the last (5x8 + 5x8 + 8) / S; per face: face output
-        # record (32); per ghost: record in and out (2x32) + ids (2i)
+        # per cell: CSR ptr (i) + K entries (i) + K face areas (s) + V (g) + the iteration's FP64
+        # start state read (5x8) + new state record (32) + ghost ptr (i), and, averaged over the S
+        # stages of an iteration, w and dt written on the last (5x8 + 8) / S; per face: face
+        # output record (32); per ghost: record in and out (2x32) + ids (2i)
         S = SCHEME["rk_level"]
-        return nint * (4 + 4 * K + 4 * K + 8 + 8 + 40 + 88.0 / S + 32 + 4) + nf * 32 + ngh * 72
+        return nint * (4 + 4 * K + 4 * K + 8 + 40 + 48.0 / S + 32 + 4) + nf * 32 + ngh * 72
     if kind == "gradient":
         if precision == 32 and K == 4:
             # FP32, 4 faces per cell (the per-entry coefficient table): per cell the 4
@@ -611,9 +610,9 @@ def run_gpu(args):
         nsteps = info["period"] * (2 * per_step * nopi - 1) + info["levels"] + 1  # of the profiled call
         roof = {"bound": "latency", "kernel": "wavefront", "achieved": None, "peak": peak, "peak_kind": peak_kind,
                 "unit": "GB/s", "frac": None, "traffic": None,
-                "note": "one persistent launch per call; a %d-iteration call is %d grid-barrier steps "
-                        "(period %d, %d levels, %d CTAs), %.2f us per step: bound by the barrier and the "
-                        "dependent loads of a step, not by HBM" %
+                "note": "one persistent launch per call; a %d-iteration call is %d steps of the level chain "
+                        "(period %d, %d levels, %d CTAs), %.2f us per step: bound by the exchange of states and "
+                        "a step's own instructions, not by HBM" %
                         (2 * per_step, nsteps, info["period"], info["levels"], info["blocks"],
                          1000.0 * kms / kcnt / nsteps)}
     else:

@@ -268,12 +268,12 @@ class Solver:
     graphs_on = False
 
     def use_wavefront(self, on=True):
-        """Sequential LocalAccTime1 as one persistent launch per call (default
-        on) or level by level, stage by stage (off); same results."""
+        """One resident launch per call for the sequential LocalAccTime1 and for
+        small meshes (default on), or launch by launch (off); same FP64 results."""
         check(_lib.load().psst_solver_use_wavefront(self._h, int(bool(on))))
 
     def set_wait_limit(self, nanoseconds):
-        """Bound of each device-side wait of the persistent launch (< 0: default)."""
+        """Bound of each device-side wait of the resident launch (< 0: default)."""
         check(_lib.load().psst_solver_set_wait_limit(self._h, int(nanoseconds)))
 
     def schedule_info(self):
