@@ -57,7 +57,8 @@ __device__ __forceinline__ bool den_ok(R b) {
         // temperature settling at 300, have a low word of ones and nothing more (and
         // settled flows are full of them: 25 instead of 20 us an iteration of 120 x 40
         // quads while they took the plain operators)
-        return (__double2loint(b) != -1 || (~__double2hiint(b) & 0xfffff) != 0) && positive_in_range<400, 400>(fabs(b));
+        return ((uint32_t)__double2loint(b) & ((uint32_t)__double2hiint(b) | 0xfff00000u)) != 0xffffffffu &&
+               positive_in_range<400, 400>(fabs(b));
     else
         return positive_in_range<60, 60>(fabsf(b));
 }
