@@ -715,7 +715,6 @@ void raise_err(psst_solver *s, const int32_t e[4], const int32_t *err_dev) {
     case 3:
         raise(PSST_ERR_NONFINITE, "non-finite residual in cell " + std::to_string(s->L.vol_of_dev[e[1]]));
     case 5:
-        s->res_dirty = true;
         raise(PSST_ERR_TIMEOUT, "a wait of the resident launch ran out (operation " + std::to_string(e[1]) +
                                     "); the state is undefined until the next psst_solver_set_state");
     default:
@@ -929,15 +928,19 @@ bool resident_run(psst_solver *s, int n_iter, Mark &&mark) {
         s->res.rows = (double *)s->dalloc_bytes(need);
         s->res_rows_cap = need;
     }
+    // a launch that gave up leaves its abort flag, arrivals and tags behind, whatever error is
+    // reported first: the buffers count as clean again only once run() has seen no error
+    bool clear = s->res_dirty;
+    s->res_dirty = true;
     for (int done = 0; done < n_iter;) {
         const int n = std::min(n_iter - done, most);
         const uint32_t stages = (uint32_t)n * (uint32_t)s->sc.rk_level;
-        if (s->res_dirty || s->res_tag > 0x7fffffffu - stages || s->res_ptag > 0x7fffffffu - (uint32_t)n) {
+        if (clear || s->res_tag > 0x7fffffffu - stages || s->res_ptag > 0x7fffffffu - (uint32_t)n) {
             for (auto p : s->res_state) ck(cudaMemsetAsync(p, 0, s->res_state_bytes, s->stream), "memset");
             if (s->res_proj) ck(cudaMemsetAsync(s->res_proj, 0, s->res_proj_bytes, s->stream), "memset");
             ck(cudaMemsetAsync(s->res.sync, 0, kWfSyncWords * sizeof(unsigned), s->stream), "memset");
             s->res_tag = s->res_ptag = s->res_arrived = 0;
-            s->res_dirty = false;
+            clear = false;
         }
         ResArgs<R> a{};
         a.g = s->g;
@@ -1016,7 +1019,8 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
     int64_t launches = 0;
     ck(cudaEventRecord(s->ev0, s->stream), "event");
     const auto count = [&](int) { ++launches; };
-    if (resident_active(s) && resident_run<R>(s, n_iter, count)) {
+    const bool resident = resident_active(s) && resident_run<R>(s, n_iter, count);
+    if (resident) {
         // one launch, which wrote every residual column
     } else if (s->use_graphs) {
         const NormFork fork(s, true);
@@ -1071,6 +1075,7 @@ void run(psst_solver *s, int n_iter, double *res_linf, double *res_l2) {
         const int32_t e[4] = {he[0], he[1], he[2], he[3]};
         raise_err(s, e, w.err);
     }
+    if (resident) s->res_dirty = false;
     float ms = 0.0f;
     ck(cudaEventElapsedTime(&ms, s->ev0, s->ev1), "event time");
     s->last_ms = ms;

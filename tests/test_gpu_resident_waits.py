@@ -1,0 +1,41 @@
+"""Waits of the resident launch that run out, and small solvers beside one another."""
+import numpy as np
+import pytest
+
+from conftest import make_case
+from supersonicflowsolver_b200 import meshgen
+from supersonicflowsolver_b200.psst import Grid, PsstError, Solver
+
+pytestmark = pytest.mark.gpu
+
+
+def test_run_out_wait_behind_another_error_leaves_nothing_behind(tmp_path):
+    """Temperatures below zero everywhere: every CTA reports its cells' state in the first stage,
+    which waits for nothing (first order, local time steps from stage-start values), so that is
+    the error of the call although every wait of the second stage then runs out. The calls after
+    it, with a good state and the usual bound, equal those of a new solver, residual columns included."""
+    m = meshgen.wedge2d(61, 23, 15.0)
+    path, d, name = make_case(tmp_path, m, max_iter=1, flux=2, order=1, lc=1, rk_level=2, mach=2.5)
+    g = Grid.read_fluent(path)
+    sc, prim = g.read_case(d, name)
+    sc.precision, sc.lc1_mode = 64, 1
+    a, b = Solver(g, sc), Solver(g, sc)
+    assert a.schedule_info()["wavefront"] and a.schedule_info()["blocks"] > 1
+    bad = prim.copy()
+    bad[g.nvol:2 * g.nvol] *= -1.0
+    a.set_state(prim)
+    a.explicit_solve(3)
+    a.set_state(bad)
+    a.set_wait_limit(0)
+    with pytest.raises(PsstError) as e:
+        a.explicit_solve(2)
+    assert e.value.status in (5, 6)  # not PSST_ERR_TIMEOUT
+    a.set_wait_limit(-1)
+    for s in (a, b):
+        s.set_state(prim)
+    for n in (3, 2):
+        la, ra = a.explicit_solve(n)
+        lb, rb = b.explicit_solve(n)
+        assert np.array_equal(la, lb) and np.array_equal(ra, rb)
+        for x, y in zip(a.get_state(with_w=True), b.get_state(with_w=True)):
+            assert np.array_equal(x, y)
