@@ -49,7 +49,9 @@
 // publication, 550 ghosts, 350 norms, 900 the loop and its barrier.
 //
 // Every wait is bounded: one longer than wait_ns sets the abort flag and
-// ERR_TIMEOUT, and every warp leaves at its next wait.
+// ERR_TIMEOUT, and every warp leaves at its next wait of 256 attempts (data that
+// arrives sooner is what it waited for). A warp that gave up forms and publishes
+// nothing from what it has.
 #pragma once
 #include <type_traits>
 
@@ -438,8 +440,9 @@ struct Lane {
 // every later shuffle would cost 230 cycles more.
 __device__ __forceinline__ bool still_waiting(bool miss, bool &ok, Waiter &wt, int where) {
     if (!__any_sync(FULL, miss)) return false;
-    ok = !__any_sync(FULL, !wt.again(where));
-    return ok;
+    const bool more = !__any_sync(FULL, !wt.again(where));
+    ok = ok && more;
+    return more;
 }
 
 // Gradient of the quad's cell. Lane j forms the products of the face at its
@@ -501,6 +504,7 @@ __device__ __forceinline__ bool res_gradient(const ResArgs<R> &a, const Lane<R, 
         do {
             if (need) w.fetch(p);
         } while (still_waiting(need && (!w.holds(tag) || a.wait_ns == 0), ok, wt, where));
+        if (!ok) return false;
         R oth[NV];
 #pragma unroll
         for (int i = 0; i < NV; ++i) oth[i] = (R)0;
@@ -566,8 +570,7 @@ __device__ __forceinline__ bool res_gradient(const ResArgs<R> &a, const Lane<R, 
             }
         }
     }
-    if (__any_sync(FULL, !ok)) return false;
-        // offsets of the quad's faces: other lanes' static data, read through L1
+    // offsets of the quad's faces: other lanes' static data, read through L1
     if (REC == 2) {
         R lim[NP];
         // with `div` as the division; false where an operand is out of lin_div's range
@@ -608,7 +611,7 @@ __device__ __forceinline__ bool res_gradient(const ResArgs<R> &a, const Lane<R, 
 #pragma unroll
             for (int t = 0; t < DIM; ++t) gr[i][t] = gr[i][t] * lim[i];
     }
-        for (int r = 0; r < rounds; ++r) {
+    for (int r = 0; r < rounds; ++r) {
         const size_t lb = (size_t)L.item * rounds + r;
         const uint4 *block = a.sc.faces + lb * FD::PIECES * kWfBlock;
         const int t0 = (int)(threadIdx.x & ~3u);
@@ -746,6 +749,7 @@ __device__ __forceinline__ bool res_stage(const ResArgs<R> &a, const Lane<R, DIM
                 miss2 = miss2 && !w2.holds(tag2);
             }
         } while (still_waiting(miss1 || missp || miss2, ok, wt, where));
+        if (!ok) return false;
         if (REC != 0 && inner && first) {
             const int lane = (int)(ids.z % kWfBlock);
             const R *there = st.proj + (size_t)((int)(ids.z / kWfBlock) % rounds) * 2 * NV * kWfBlock + lane;
@@ -804,7 +808,7 @@ __device__ __forceinline__ bool res_stage(const ResArgs<R> &a, const Lane<R, DIM
                 lin_flux<R, DIM, 2>(rr, f, a.gas, edge, flow, exact);
             else
                 lin_flux<R, DIM, 3>(rr, f, a.gas, edge, flow, exact);
-            if (!exact && ok && (bits & kFaceValid)) {
+            if (!exact && (bits & kFaceValid)) {
                 PlainFace<R, DIM, REC, LIM> pf;
                 pf.r[0] = side ? oth : own;
                 pf.r[1] = side ? own : oth;
@@ -884,7 +888,6 @@ __device__ __forceinline__ bool res_stage(const ResArgs<R> &a, const Lane<R, DIM
                 }
         }
     }
-        if (__any_sync(FULL, !ok)) return false;
     if (a.lc == 2) {
 #pragma unroll
         for (int d = 0; d < DIM; ++d) den += (fabs(own.u[d]) + cc) * area[d] * (R)0.5;

@@ -1,4 +1,8 @@
 """Waits of the resident launch that run out, and small solvers beside one another."""
+import ctypes
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -39,3 +43,46 @@ def test_run_out_wait_behind_another_error_leaves_nothing_behind(tmp_path):
         assert np.array_equal(la, lb) and np.array_equal(ra, rb)
         for x, y in zip(a.get_state(with_w=True), b.get_state(with_w=True)):
             assert np.array_equal(x, y)
+
+
+HARNESS = r"""
+#include "resident.cuh"
+using namespace psst;
+// One warp: a wait that runs out (its limit is 1 ns, 4096 attempts at most), then a wait that ends after one
+// attempt. out[0], out[1]: whether the operation may go on after each.
+__global__ void k(unsigned *sync, int32_t *err, int *out) {
+    bool ok = true;
+    Waiter first{sync, err, 1, 0, 0u};
+    for (int i = 0; i < 4096 && still_waiting(true, ok, first, 0); ++i) {}
+    if (threadIdx.x == 0) out[0] = ok;
+    Waiter second{sync, err, 1000000000, 0, 0u};
+    for (int i = 0; i < 2 && still_waiting(i == 0, ok, second, 0); ++i) {}
+    if (threadIdx.x == 0) out[1] = ok;
+}
+extern "C" int run(int *out) {
+    unsigned *sync;
+    int32_t *err;
+    int *o;
+    if (cudaMalloc(&sync, kWfSyncWords * 4) || cudaMalloc(&err, 16) || cudaMalloc(&o, 8)) return 1;
+    cudaMemset(sync, 0, kWfSyncWords * 4);
+    cudaMemset(err, 0, 16);
+    k<<<1, 32>>>(sync, err, o);
+    const int e = cudaMemcpy(out, o, 8, cudaMemcpyDeviceToHost);
+    cudaFree(sync), cudaFree(err), cudaFree(o);
+    return e;
+}
+"""
+
+
+def test_a_wait_given_up_stays_given_up(tmp_path):
+    """Cells of more than four faces wait once per four: a later wait that is met does not take back
+    that an earlier one ran out."""
+    src, lib = tmp_path / "h.cu", str(tmp_path / "h.so")
+    src.write_text(HARNESS)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run(["nvcc", "-std=c++17", "-O3", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-I", os.path.join(root, "supersonicflowsolver_b200", "csrc"), "-I", os.path.join(root, "include"),
+                    "-shared", "-Xcompiler", "-fPIC", str(src), "-o", lib], check=True)
+    out = (ctypes.c_int * 2)()
+    assert ctypes.CDLL(lib).run(out) == 0
+    assert list(out) == [0, 0]
