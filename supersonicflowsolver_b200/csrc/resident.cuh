@@ -211,8 +211,9 @@ __device__ __forceinline__ Prim<R, DIM> from_record(const Record<R, DIM + 3> &w)
 // at this position of the face-loop order, -1: no such face; nb2 across the face
 // at the same position of the cell's own order), the lane record of the same face
 // in the cell across (kFaceLocal: a cell of the same item), flags, and the fields n, S | off (the face's reconstruction
-// offset on this side), g (Green-Gauss: signed S / V, beta; least squares: the
-// weights of nb2) | n2, S2 (of nb2's face). Kept in 16-byte pieces, piece-major
+// offset on this side), g (Green-Gauss: signed S / V, beta, in FP32 the weight of
+// the cell across and signed S n / V; least squares: the weights of nb2) | n2, S2
+// (of nb2's face). Kept in 16-byte pieces, piece-major
 // over the lanes, so that a warp's load is one run of 512 bytes; formed once by
 // k_res_build from the grid's own arrays with their arithmetic.
 constexpr uint32_t kFaceSide = 1, kFaceInner = 2, kFaceLow = 4, kFaceSame = 8, kFaceValid = 16, kFaceLocal = 32;
@@ -223,6 +224,7 @@ struct FaceData {
     static constexpr int OG = (DIM + 3 + PER - 1) / PER;         // pieces of off, g
     static constexpr int OFFP = (DIM + PER - 1) / PER;           // the first of them: off
     static constexpr int PIECES = 1 + 2 * NS + OG;
+    static_assert(sizeof(R) == 8 || 2 * DIM + 1 <= OG * PER, "off and the FP32 Green-Gauss coefficients");
     // pieces [A, A + N) after the ids of lane `t` of a face block, as R values
     template <int A, int N>
     static __device__ __forceinline__ void fields(const uint4 *block, int t, R *out) {
@@ -277,10 +279,15 @@ __global__ void __launch_bounds__(kWfBlock) k_res_build(DevGrid g, int rec, int 
         }
         ns[DIM] = (R)fr.S;
         ns2[DIM] = (R)fr2.S;
-        if (grad == 1) {
-            const R gp = EXACT ? (R)(fr.S / V) : (R)(fr.S * (1.0 / V));
+        if (grad == 1 && EXACT) {
+            const R gp = (R)(fr.S / V);
             og[DIM] = side ? gp : -gp;
             og[DIM + 1] = (R)g.beta[ent >> 1];
+        } else if (grad == 1) {  // the values of the gradient pass's table (build_gradient_coefficients)
+            const double sv = (side ? 1.0 : -1.0) * (fr.S / V), beta = g.beta[ent >> 1];
+            og[DIM] = (R)(side ? beta : 1.0 - beta);
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) og[DIM + 1 + k] = (R)(sv * fr.n[k]);
         } else if (grad == 2) {  // as gradient_cell forms them (psstGradCalculation.cpp:268-368)
             R lr[7], diff[DIM], w = (R)0;
 #pragma unroll
@@ -523,33 +530,61 @@ __device__ __forceinline__ bool res_gradient(const ResArgs<R> &a, const Lane<R, 
                 for (int i = 0; i < NV; ++i) oth[i] = pvar<R, DIM>(x, i);
             }
         }
-        const bool side = bits & kFaceSide;
-        const R coef = f2[DIM], beta = f2[DIM + 1];
-        R tv[NV];
+        if constexpr (sizeof(R) == 4) {
+            // as gradient_cell_table: face values in one rounding, summed by fused products
+            // with the table's coefficients (products rounded here and then added: errors
+            // of u 6% larger after 30 iterations of 3000 tets)
+            R tv[NV], d[DIM];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const R av = pvar<R, DIM>(own, i);
-            if (gg) {
-                const R phi0 = side ? oth[i] : av, phi1 = side ? av : oth[i];
-                tv[i] = (beta * phi0 + ((R)1 - beta) * phi1) * coef;
-            } else {
-                tv[i] = oth[i] - av;
+            for (int i = 0; i < NV; ++i) {
+                const R av = pvar<R, DIM>(own, i);
+                tv[i] = gg ? fmaf(f2[DIM], oth[i] - av, av) : oth[i] - av;
             }
-        }
 #pragma unroll
-        for (int t = 0; t < DIM; ++t) {
-            const R d = gg ? f1[t] : f2[DIM + t];
-            R x[4], x4 = (R)0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) x[i] = tv[i] * d;
-            if (NP == 2) x4 = tv[NV - 1] * d;
-            quad_transpose(x, q);
+            for (int t = 0; t < DIM; ++t) d[t] = gg ? f2[DIM + 1 + t] : f2[DIM + t];
+            const R tv4 = tv[NV - 1];
+            quad_transpose(tv, q);
 #pragma unroll
             for (int jj = 0; jj < 4; ++jj) {
-                const R y4 = NP == 2 ? __shfl_sync(FULL, x4, qb + jj) : (R)0;
-                if ((vq >> jj) & 1u) {
-                    gr[0][t] += x[jj];
-                    if (NP == 2) gr[NP - 1][t] += y4;
+                const R y4 = NP == 2 ? __shfl_sync(FULL, tv4, qb + jj) : (R)0;
+#pragma unroll
+                for (int t = 0; t < DIM; ++t) {
+                    const R dj = __shfl_sync(FULL, d[t], qb + jj);
+                    if ((vq >> jj) & 1u) {
+                        gr[0][t] = fmaf(tv[jj], dj, gr[0][t]);
+                        if (NP == 2) gr[NP - 1][t] = fmaf(y4, dj, gr[NP - 1][t]);
+                    }
+                }
+            }
+        } else {
+            const bool side = bits & kFaceSide;
+            const R coef = f2[DIM], beta = f2[DIM + 1];
+            R tv[NV];
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const R av = pvar<R, DIM>(own, i);
+                if (gg) {
+                    const R phi0 = side ? oth[i] : av, phi1 = side ? av : oth[i];
+                    tv[i] = (beta * phi0 + ((R)1 - beta) * phi1) * coef;
+                } else {
+                    tv[i] = oth[i] - av;
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < DIM; ++t) {
+                const R d = gg ? f1[t] : f2[DIM + t];
+                R x[4], x4 = (R)0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[i] = tv[i] * d;
+                if (NP == 2) x4 = tv[NV - 1] * d;
+                quad_transpose(x, q);
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) {
+                    const R y4 = NP == 2 ? __shfl_sync(FULL, x4, qb + jj) : (R)0;
+                    if ((vq >> jj) & 1u) {
+                        gr[0][t] += x[jj];
+                        if (NP == 2) gr[NP - 1][t] += y4;
+                    }
                 }
             }
         }

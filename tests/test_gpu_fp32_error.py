@@ -6,6 +6,10 @@ import subprocess
 import numpy as np
 import pytest
 
+from conftest import make_case
+from supersonicflowsolver_b200 import meshgen
+from supersonicflowsolver_b200.psst import Grid, Solver
+
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -103,3 +107,28 @@ def test_energy_flux_rounds_the_enthalpy_once(face_lib, flux, rec):
         vs = (u[d] * u[d] + vs).astype(f32).astype(np.float64)
     H = (np.float64(f32(1004.5)) * T + 0.5 * vs).astype(f32)
     assert np.array_equal(out[:, 4], out[:, 3] * H)
+
+
+@pytest.mark.parametrize("mesh", ["quads", "shuffled", "tets"])
+def test_resident_gradient_has_the_bits_of_the_pass(tmp_path, mesh):
+    """Four faces a cell, FP32: the gradients that the resident launch forms from a state are those of the
+    gradient pass (one fused product a face, coefficients rounded once)."""
+    m = {"quads": lambda: meshgen.wedge2d(61, 23, 15.0), "tets": lambda: meshgen.wedge3d(9, 5, 3, 12.0, tets=True),
+         "shuffled": lambda: meshgen.wedge2d(30, 10, 15.0, jitter=0.15, seed=3, shuffle_seed=1, interior_first=True)}[mesh]()
+    path, d, name = make_case(tmp_path, m, max_iter=4, flux=3, order=2, limiter=3, lc=1, mach=3.0 if m.dim == 3 else 2.5)
+    g = Grid.read_fluent(path)
+    sc, prim = g.read_case(d, name)
+    sc.precision, sc.lc1_mode = 32, 1
+    a, b = Solver(g, sc), Solver(g, sc)
+    b.use_wavefront(False)
+    assert a.schedule_info()["wavefront"]
+    b.set_state(prim)
+    b.explicit_solve(3)
+    start = b.get_state()  # FP32 values: both solvers start from the same bits
+    got = []
+    for s in (a, b):
+        s.set_state(start)
+        s.explicit_solve(1)
+        got.append([s.get(k) for k in ("grad_p", "grad_T", "grad_u")])
+    for x, y in zip(*got):
+        assert np.abs(y).max() > 0 and np.array_equal(x, y)
