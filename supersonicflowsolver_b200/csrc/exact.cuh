@@ -16,7 +16,9 @@
 //    b q) y rounds to the correctly rounded quotient. y comes from the
 //    approximate reciprocal by a cubic Newton step and a quadratic one, which
 //    rounds it correctly unless b's mantissa is all ones (den_ok excludes it);
-//    a y, at most 1.5 ulp off, is corrected twice.
+//    a y, at most 1.5 ulp off, is corrected twice. A zero numerator keeps its sign
+//    over a positive b (the residual is formed negated, b q - a, whose exact zero is
+//    +0 and adds nothing to a -0); over a negative one the zero's sign is open.
 //  * square root: a cubic step from the approximate reciprocal square root gives
 //    a root s within one ulp; the signs of x - s s+ and x - s s- (s+, s- its
 //    neighbours; Tuckerman's test, in the same paper) say which of the three is
@@ -25,8 +27,11 @@
 // caller checks its operands (in_range, zero_or_in_range, den_ok) and takes the
 // plain operators otherwise.
 //
-// FP32: the approximate reciprocal (square root) with one residual correction,
-// within 0.51 ulp of the exact value. rn_div is the rounded quotient, as above.
+// FP32: the approximate reciprocal (square root) with one residual correction. The
+// quotient's correction is itself good to 2^-22, so it is the rounded one but for
+// exact values within 2^-21 ulp of a rounding boundary; the root is within 0.51 ulp
+// of the exact value. rn_div corrects the reciprocal too: the rounded quotient, as
+// above.
 #pragma once
 #include <cstdint>
 
@@ -80,20 +85,23 @@ __device__ __forceinline__ float lin_recip(float b) {
 // a / b given y = lin_recip(b)
 __device__ __forceinline__ double lin_quot(double a, double b, double y) {
     double t = a * y;
-    t = fma(fma(-b, t, a), y, t);
-    return fma(fma(-b, t, a), y, t);
+    t = fma(-fma(b, t, -a), y, t);
+    return fma(-fma(b, t, -a), y, t);
 }
 __device__ __forceinline__ float lin_quot(float a, float b, float y) {
     const float t = a * y;
-    return fmaf(fmaf(-b, t, a), y, t);
+    return fmaf(-fmaf(b, t, -a), y, t);
 }
 template <typename R>
 __device__ __forceinline__ R lin_div(R a, R b) {
     return lin_quot(a, b, lin_recip(b));
 }
-// the same with the reciprocal corrected first, which rounds it correctly:
-// the bits of a / b for 2^-126 <= 1 / b and 2^-100 <= |a|, |a / b| (smaller
-// quantities lose bits of the residual), and for a = 0 up to the sign of a -0
+// the same with the reciprocal corrected first, which rounds it correctly (of 2 -
+// 2^-23 and its like, which the correction could leave at a tie, the approximate
+// reciprocal is the rounded one on sm_100): the bits of a / b while 1 / b, a / b and
+// the residual b q - a, some 2^-24 of a, are normal numbers, and for a = 0. activate()
+// (mlp_net.cuh) has 1 <= b < 2^126 and |a| < 87: b is 2 to all bits where |a| is too
+// small for a normal residual, and the halves are exact.
 __device__ __forceinline__ float rn_div(float a, float b) {
     float y = lin_recip(b);
     y = fmaf(fmaf(-b, y, 1.0f), y, y);
