@@ -448,6 +448,12 @@ psst_status psst_mlp_train_step(psst_mlp *m, const float *x, const float *t, int
  * stream must be complete before a call, and y of psst_mlp_forward is
  * complete only in `stream`'s order. */
 psst_status psst_mlp_set_stream(psst_mlp *m, void *stream);
+/* Bound of each mbarrier wait of the network's kernels, in polls (< 0: the
+ * default, about a second or more; 0: each gives up at once). A wait that runs
+ * out makes the call return PSST_ERR_TIMEOUT once the MMAs and copies in flight
+ * are done; parameters, Adam state and step stay as they were (psst_mlp_forward:
+ * y is undefined). Used to test that path. */
+psst_status psst_mlp_set_wait_polls(psst_mlp *m, int64_t polls);
 void psst_mlp_destroy(psst_mlp *m);
 
 /* The tensor-core GEMM on its own: D[z][m][n] = sum over k of split z of

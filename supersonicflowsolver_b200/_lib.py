@@ -32,8 +32,8 @@ EXPORTED = [
     "psst_solver_set_stop_rule", "psst_solver_case_status", "psst_solver_save_checkpoint",
     "psst_solver_load_checkpoint", "psst_solver_run_to_stop",
     "psst_mlp_create", "psst_mlp_param_count", "psst_mlp_get_params", "psst_mlp_set_params", "psst_mlp_forward",
-    "psst_mlp_gradients", "psst_mlp_train_step", "psst_mlp_set_stream", "psst_mlp_destroy", "psst_tc_gemm_bf16",
-    "psst_tc_gemm_bf16_wait", "psst_tc_gemm_bf16_time",
+    "psst_mlp_gradients", "psst_mlp_train_step", "psst_mlp_set_stream", "psst_mlp_set_wait_polls", "psst_mlp_destroy",
+    "psst_tc_gemm_bf16", "psst_tc_gemm_bf16_wait", "psst_tc_gemm_bf16_time",
 ]
 
 
@@ -141,6 +141,7 @@ def load():
         "psst_mlp_gradients": (I, [P, P, P, I, P, ctypes.POINTER(ctypes.c_float)]),
         "psst_mlp_train_step": (I, [P, P, P, I, ctypes.c_float, ctypes.POINTER(ctypes.c_float)]),
         "psst_mlp_set_stream": (I, [P, P]),
+        "psst_mlp_set_wait_polls": (I, [P, I64]),
         "psst_mlp_destroy": (None, [P]),
         "psst_tc_gemm_bf16": (I, [P, I64, I64, P, I64, I64, I, I, I, I, P, I64, P]),
         "psst_tc_gemm_bf16_wait": (I, [P, I64, I64, P, I64, I64, I, I, I, I, P, I64, P, I64]),

@@ -534,6 +534,7 @@ struct psst_mlp {
     float *dy = nullptr, *lpart = nullptr, *part = nullptr;
     NetMaps maps{};
     int *status = nullptr;  // error word, loss
+    unsigned wait_polls = kWaitLimit;
     std::vector<void *> allocs, ws;
     ~psst_mlp() {
         cudaSetDevice(device);
@@ -769,7 +770,7 @@ float finish(psst_mlp *m) {
     ck(cudaStreamSynchronize(m->stream), "stream sync");
     if (status[0]) {
         ck(cudaMemsetAsync(m->status, 0, sizeof(int), m->stream), "memset");
-        raise(PSST_ERR_TIMEOUT, "tensor-core GEMM: an mbarrier wait ran out");
+        raise(PSST_ERR_TIMEOUT, "network kernels: an mbarrier wait ran out");
     }
     float loss;
     std::memcpy(&loss, status + 1, sizeof loss);
@@ -781,7 +782,7 @@ void chain(psst_mlp *m, const float *x, const float *t, int B, float *y) {
     static thread_local unsigned long long done_devices = 0;
     smem_attribute(k_net<TRAIN>, net_smem<TRAIN>(), done_devices);
     k_net<TRAIN><<<nb(B, kTileM), kNetThreads, net_smem<TRAIN>(), m->stream>>>(
-        m->maps, NetArgs{m->net, m->p, x, t, y, m->dy, m->lpart, B, m->status});
+        m->maps, NetArgs{m->net, m->p, x, t, y, m->dy, m->lpart, B, m->status, m->wait_polls});
 }
 
 // Forward and backward pass, weight gradients, and their sums over the batch:
@@ -796,7 +797,7 @@ void gradients(psst_mlp *m, const float *x, const float *t, int B, const AdamArg
         const int n = std::min(splits - s0, kSplitsMax);
         const int units = n * kWgradUnits;
         k_wgrad<<<std::min(units, m->sms), kWgradThreads, kWgradSmem, s>>>(
-            m->maps, WgradArgs{m->net, m->dy, m->part, B, s0, units, m->status});
+            m->maps, WgradArgs{m->net, m->dy, m->part, B, s0, units, m->status, m->wait_polls});
         const LossArgs loss{m->lpart, (int)nb(B, kTileM), 1.0 / ((double)kOut * B), m->status};
         if (adam && s0 + n == splits)
             k_reduce<true><<<nb(n4), 256, 0, s>>>(m->part, n, n4, s0 == 0, m->g, *adam, loss);
@@ -931,6 +932,13 @@ extern "C" psst_status psst_mlp_train_step(psst_mlp *m, const float *x, const fl
     const float l = finish(m);
     m->step += 1;
     if (loss) *loss = l;
+    MLP_END
+}
+
+extern "C" psst_status psst_mlp_set_wait_polls(psst_mlp *m, int64_t polls) {
+    MLP_BEGIN
+    if (!m) raise(PSST_ERR_ARG, "psst_mlp_set_wait_polls: null network");
+    m->wait_polls = polls < 0 || polls > (int64_t)kWaitLimit ? kWaitLimit : (unsigned)polls;
     MLP_END
 }
 

@@ -71,6 +71,7 @@ struct NetArgs {
     float *loss_part;    // per CTA, sum of (y - t)^2
     int B;
     int *err;
+    unsigned wait_polls;  // bound of every wait but the final ones (kWaitLimit; 0: each gives up at once)
 };
 
 constexpr int kEpiWarps = 16, kNetThreads = 32 * (kEpiWarps + 2);
@@ -91,8 +92,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 }
 // mbar_wait of a whole warp, polled in step: lanes that left a loop of their own one
 // by one would stay apart for what follows.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned phase) {
-    for (unsigned i = 0; i < kWaitLimit; ++i)
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned phase, unsigned limit) {
+    for (unsigned i = 0; i < limit; ++i)
         if (__all_sync(0xffffffffu, mbar_wait(bar, phase, 1))) return true;
     return false;
 }
@@ -176,8 +177,10 @@ __device__ __forceinline__ void unpack8(const uint4 &q, float *v) {
 // all MMAs of the step done and the copies out of the operand buffers read
 // (a commit and an arrival); wfull / wempty per weight stage; zfull[c],
 // pre-activation chunk c loaded.
-// A wait that runs out ends its role; the others' waits then run out too, the
-// issuing threads see their MMAs and copies finish, and the CTA leaves with *err.
+// A wait that runs out ends its role; the others' waits then run out too, and the
+// CTA leaves with *err. Whatever the others do, each issuing thread sees its own MMAs
+// and copies finish before the CTA's last barrier: a role that gave up no longer
+// waits for them, and none may be in flight when the CTA gives its memory back.
 template <bool TRAIN>
 __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ NetMaps maps,
                                                         const __grid_constant__ NetArgs a) {
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ 
                 const int l = back ? 2 * kHidden - 1 - s : s, nch = s == 0 ? 2 : 4;
                 for (int c = 0; c < nch; ++c, ++n) {
                     const int b = n % kWStages, use = n / kWStages;
-                    if (use > 0 && !(ok = mbar_wait(&wempty[b], (unsigned)(use - 1) & 1u))) break;
+                    if (use > 0 && !(ok = mbar_wait(&wempty[b], (unsigned)(use - 1) & 1u, a.wait_polls))) break;
                     mbar_expect_tx(&wfull[b], kWeightChunk);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
@@ -231,16 +234,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ 
                                  64 * (back ? c : j), &wfull[b]);
                 }
             }
-            if (!ok)  // let the copies in flight land
-                for (int i = max(0, n - kWStages); i < n; ++i)
-                    mbar_wait(&wfull[i % kWStages], (unsigned)(i / kWStages) & 1u);
+            for (int i = max(0, n - kWStages); i < n; ++i)  // the last copies land
+                mbar_wait(&wfull[i % kWStages], (unsigned)(i / kWStages) & 1u);
         }
     } else if (warp == kEpiWarps) {
         if (lane == 0) {  // MMAs and activation copies
             int n = 0, nz = 0;
             unsigned hph = 0;  // bit c: phase of hready[c]
             auto wait_h = [&](int c) {
-                const bool r = mbar_wait(&hready[c], (hph >> c) & 1u);
+                const bool r = mbar_wait(&hready[c], (hph >> c) & 1u, a.wait_polls);
                 hph ^= 1u << c;
                 return r;
             };
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ 
                         }
                         bulk_commit();
                     }
-                    if (!(ok = mbar_wait(&wfull[b], (unsigned)(n / kWStages) & 1u))) break;
+                    if (!(ok = mbar_wait(&wfull[b], (unsigned)(n / kWStages) & 1u, a.wait_polls))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = smem_u32(hbuf + c * kActChunk), sb = smem_u32(wbuf + b * kWeightChunk);
 #pragma unroll
@@ -309,13 +311,11 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ 
                 bulk_commit();
                 bulk_wait();
             }
-            if (!ok) {  // let what is in flight finish
-                for (int i = max(0, n - kWStages); i < n; ++i)
-                    mbar_wait(&wempty[i % kWStages], (unsigned)(i / kWStages) & 1u);
-                for (int i = max(0, nz - 4); i < nz; ++i) mbar_wait(&zfull[i & 3], (unsigned)(i >> 2) & 1u);
-                bulk_commit();
-                bulk_wait();
-            }
+            // the last MMAs and copies finish
+            for (int i = max(0, n - kWStages); i < n; ++i) mbar_wait(&wempty[i % kWStages], (unsigned)(i / kWStages) & 1u);
+            for (int i = max(0, nz - 4); i < nz; ++i) mbar_wait(&zfull[i & 3], (unsigned)(i >> 2) & 1u);
+            bulk_commit();
+            bulk_wait();
         }
     } else {
         const int row = 32 * (warp & 3) + lane, grow = row0 + row, grp = warp >> 2;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ 
         const bool in = grow < a.B;
         unsigned aph = 0, zph = 0;
         auto wait_acc = [&] {
-            const bool r = mbar_wait_warp(&accfull, aph);
+            const bool r = mbar_wait_warp(&accfull, aph, a.wait_polls);
             aph ^= 1u;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             return r;
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net(const __grid_constant__ 
                     // the factors of a chunk are formed ahead of its product: the first under the MMAs
                     float v[16];
                     auto factors = [&](int c) {
-                        if (!mbar_wait_warp(&zfull[c], zph)) return false;
+                        if (!mbar_wait_warp(&zfull[c], zph, a.wait_polls)) return false;
 #pragma unroll
                         for (int u = 0; u < 2; ++u)
                             unpack8(*act_unit(zbuf + c * kActChunk, row, 2 * grp + u), v + 8 * u);
@@ -512,6 +512,7 @@ struct WgradArgs {
     float *part;
     int B, split0, units;
     int *err;
+    unsigned wait_polls;  // as in NetArgs
 };
 
 __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad(const __grid_constant__ NetMaps maps,
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad(const __grid_constan
                 const CUtensorMap *mb = t.l == 0 ? &maps.f : &maps.h[t.l - 1];
                 for (int c = 0; c < t.nchunks; ++c, ++n) {
                     const int b = n % kWgradStages, row = t.b0 + 64 * c;
-                    if (n >= kWgradStages && !(ok = mbar_wait(&empty[b], phase_of(n) ^ 1u))) break;
+                    if (n >= kWgradStages && !(ok = mbar_wait(&empty[b], phase_of(n) ^ 1u, a.wait_polls))) break;
                     unsigned char *sa = smem + b * kWgradStage, *sb = sa + kActChunk;
                     const uint32_t bb = (uint32_t)(t.din / 64) * kBoxBytes;
                     if (t.l == kHidden) {
@@ -586,8 +587,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad(const __grid_constan
                     for (int j = 0; j < t.din / 64; ++j) tma_load(sb + j * kBoxBytes, mb, 64 * j, row, &full[b]);
                 }
             }
-            if (!ok)  // let the copies in flight land
-                for (int i = max(0, n - kWgradStages); i < n; ++i) mbar_wait(full_of(i), phase_of(i));
+            for (int i = max(0, n - kWgradStages); i < n; ++i) mbar_wait(full_of(i), phase_of(i));  // the last copies land
         }
     } else if (warp == kWgradEpi + kWgradSum + 1) {
         if (lane == 0) {  // MMAs
@@ -595,11 +595,11 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad(const __grid_constan
             for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const Unit t = decode(u);
                 const uint32_t acc = tmem + (uint32_t)(k & 1) * kWidth;
-                if (t.l < kHidden && k >= 2 && !(ok = mbar_wait(&tempty[k & 1], (unsigned)((k >> 1) - 1) & 1u))) break;
+                if (t.l < kHidden && k >= 2 && !(ok = mbar_wait(&tempty[k & 1], (unsigned)((k >> 1) - 1) & 1u, a.wait_polls))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int c = 0; c < t.nchunks; ++c, ++n) {
                     const int b = n % kWgradStages;
-                    if (!(ok = mbar_wait(&full[b], phase_of(n)))) break;
+                    if (!(ok = mbar_wait(&full[b], phase_of(n), a.wait_polls))) break;
                     if (t.l == kHidden) {
                         mbar_arrive(&empty[b]);
                         continue;
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad(const __grid_constan
             float s = 0.0f, s0[kOut] = {}, s1[kOut] = {}, sb[kOut] = {};
             for (int c = 0; c < t.nchunks; ++c, ++n) {
                 const int b = n % kWgradStages;
-                if (!(ok = mbar_wait_warp(&full[b], phase_of(n)))) break;
+                if (!(ok = mbar_wait_warp(&full[b], phase_of(n), a.wait_polls))) break;
                 const unsigned char *sa = smem + b * kWgradStage;
                 if (t.l < kHidden) {
                     const unsigned char *box = sa + (j >> 6) * kBoxBytes + (j & 7) * 2;
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_wgrad(const __grid_constan
             const Unit t = decode(u);
             if (t.l == kHidden) continue;
             const uint32_t acc = tmem + ((uint32_t)r0 << 16) + (uint32_t)(k & 1) * kWidth;
-            if (!(ok = mbar_wait_warp(&tfull[k & 1], (unsigned)(k >> 1) & 1u))) break;
+            if (!(ok = mbar_wait_warp(&tfull[k & 1], (unsigned)(k >> 1) & 1u, a.wait_polls))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int half = t.din / 2;
             for (int c0 = 0; c0 < half; c0 += 32) {

@@ -99,6 +99,10 @@ class MLP:
     def set_stream(self, stream_ptr):
         check(_lib.load().psst_mlp_set_stream(self._h, ctypes.c_void_p(stream_ptr)))
 
+    def set_wait_polls(self, polls):
+        """Bound of each device-side wait of the network's kernels (< 0: default)."""
+        check(_lib.load().psst_mlp_set_wait_polls(self._h, int(polls)))
+
     def close(self):
         if getattr(self, "_h", None):
             _lib.load().psst_mlp_destroy(self._h)
