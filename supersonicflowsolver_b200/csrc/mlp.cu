@@ -913,7 +913,10 @@ extern "C" psst_status psst_mlp_gradients(psst_mlp *m, const float *x, const flo
     ensure_ws(m, B);
     gradients(m, x, t, B, nullptr);
     const float l = finish(m);
-    if (grads) ck(cudaMemcpy(grads, m->g, m->net.nparam * sizeof(float), cudaMemcpyDeviceToHost), "copy");
+    if (grads) {
+        ck(cudaMemcpyAsync(grads, m->g, m->net.nparam * sizeof(float), cudaMemcpyDeviceToHost, m->stream), "copy");
+        ck(cudaStreamSynchronize(m->stream), "stream sync");
+    }
     if (loss) *loss = l;
     MLP_END
 }

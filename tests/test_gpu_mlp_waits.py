@@ -1,4 +1,4 @@
-"""Waits of the network's kernels that run out."""
+"""Waits of the network's kernels that run out, and waits that a call does not have."""
 import numpy as np
 import pytest
 
@@ -40,3 +40,26 @@ def test_waits_that_run_out_are_reported_and_change_nothing(n):
         assert net.train_step(x, t, 1e-3) == ref.train_step(x, t, 1e-3)
     assert np.array_equal(net.params(), ref.params())
     assert torch.equal(net.forward(x), ref.forward(x))
+
+
+def test_gradients_wait_for_nothing_on_the_default_stream():
+    """On a stream of its own a call does not wait for what the legacy default stream has to do (a spin
+    of some 200 ms, against a call of a millisecond)."""
+    from supersonicflowsolver_b200.mlp import MLP
+
+    if not hasattr(torch.cuda, "_sleep"):
+        pytest.skip("torch.cuda._sleep not available")
+    net = MLP(seed=2)
+    x, t = (torch.from_numpy(q).cuda() for q in data(300, 4))
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        g0, l0 = net.gradients(x, t)
+    torch.cuda._sleep(400_000_000)
+    done = torch.cuda.Event()
+    done.record()
+    with torch.cuda.stream(side):
+        g1, l1 = net.gradients(x, t)
+    assert not done.query()
+    assert np.array_equal(g0, g1) and l0 == l1
+    torch.cuda.synchronize()
