@@ -396,9 +396,24 @@ psst_status psst_solver_case_residuals(psst_solver *s, int n_iter, double *out);
  *    reference's in-loop order (psstFiniteVolumeGrid.cpp:317-323) as a wavefront,
  *    operations of many iterations overlapping along the level chain;
  *  - the parallel modes on single grids small enough for one wave of CTAs.
- * FP64 results are bit-identical to the launch-by-launch form (on == 0, also the
- * path of the stage-by-stage API, of psst_solver_profile and of merged grids).
- * Calls are not captured as CUDA graphs in this mode. */
+ * FP64 states and L-inf columns are bit-identical to the launch-by-launch form (on
+ * == 0, also the path of the stage-by-stage API, of psst_solver_profile and
+ * psst_solver_autotune, and of merged grids); the RMS column is added up in another
+ * order. FP32 results of the two forms differ by roundings, so an FP32 case can
+ * differ by them between a solver of its own and a merged grid, and between devices
+ * of different SM counts ("small enough" depends on it); errors against FP64 are
+ * the same. Calls are not captured as CUDA graphs in this mode. A call of thousands
+ * of iterations takes up to 256 MB of device memory for its norm rows.
+ *
+ * Several solvers on threads or streams of their own: launches that fit the device
+ * together run together, others one after the other. Small solvers gain in any
+ * number, those whose launch takes more than half of the device lose from three or
+ * four on, where passes of many solvers interleave better; on == 0, or one merged
+ * grid, is the faster form there. us an iteration and solver at 1, 2, 4 threads,
+ * resident / passes (HLLC MUSCL RK4 quads): FP64 60 x 20 19.6 9.9 5.2 / 48.4 26.0
+ * 13.7; 120 x 40 20.4 20.3 20.2 / 49.2 26.7 14.0; 160 x 60 31.4 32.1 32.2 / 49.2
+ * 26.7 15.3; FP32 120 x 40 16.5 9.1 6.5 / 33.6 18.2 9.8; 180 x 60 18.4 19.0 19.1 /
+ * 33.3 18.3 10.1; 240 x 80 28.7 28.2 28.2 / 34.8 19.5 11.0. */
 psst_status psst_solver_use_wavefront(psst_solver *s, int on);
 
 /* Bound of each device-side wait of the resident launch (for other cells'

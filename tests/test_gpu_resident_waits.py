@@ -86,3 +86,42 @@ def test_a_wait_given_up_stays_given_up(tmp_path):
     out = (ctypes.c_int * 2)()
     assert ctypes.CDLL(lib).run(out) == 0
     assert list(out) == [0, 0]
+
+
+def test_solvers_on_threads_of_their_own(tmp_path):
+    """Four solvers, two of them with launches of more than half of the device's CTAs and one
+    sequential, step at the same time: nothing waits for another's launch beyond its end, and
+    every result is that of the solver alone."""
+    import threading
+
+    cases = []
+    for i, (nx, ny, bits, mode) in enumerate([(120, 40, 64, 1), (180, 60, 32, 1), (60, 20, 64, 1), (60, 20, 64, 0)]):
+        p = tmp_path / str(i)
+        p.mkdir()
+        path, d, name = make_case(p, meshgen.wedge2d(nx, ny, 12.0), max_iter=1, flux=3, order=2, limiter=4, lc=1)
+        g = Grid.read_fluent(path)
+        sc, prim = g.read_case(d, name)
+        sc.precision, sc.lc1_mode = bits, mode
+        s = Solver(g, sc)
+        assert s.schedule_info()["wavefront"]
+        s.set_wait_limit(2_000_000_000)
+        cases.append((s, prim))
+
+    def steps(s, prim, out):
+        s.set_state(prim)
+        out += [s.explicit_solve(20) for _ in range(10)]
+        out.append((s.get_state(),))
+
+    alone, beside = [[] for _ in cases], [[] for _ in cases]
+    for (s, prim), out in zip(cases, alone):
+        steps(s, prim, out)
+    threads = [threading.Thread(target=steps, args=c + (out,)) for c, out in zip(cases, beside)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, beside):
+        assert len(a) == len(b) == 11
+        for x, y in zip(a, b):
+            for v, w in zip(x, y):
+                assert np.array_equal(v, w)
