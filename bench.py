@@ -512,8 +512,8 @@ def gemm_throughput():
     gemm_flops = 2.0 * 16384 * (3 * (256 * 128 + 4 * 256 * 256) - 256 * 128)
     out["mlp_train_step_16384"] = {"ms": step_ms, "gemm_tflops_effective": gemm_flops / (step_ms * 1e-3) / 1e12,
                                    "note": "wall time per step (it reads the loss back, so each step waits for "
-                                           "its kernels); 14 tensor-core GEMMs plus features, output layer, "
-                                           "reductions and Adam"}
+                                           "its kernels): three kernels, with 14 layer products on the tensor "
+                                           "cores, features, output layer, sums and Adam"}
     net.close()
     return out
 
@@ -545,10 +545,10 @@ def run_gpu(args):
     # one step: one iteration, or a whole run (the published solve; the 2000-iteration case)
     per_step = int(sc.max_iter) if shipped else int(wl.get("step_iters", 1))
     whole = per_step > 1  # sequential LocalAccTime1: one persistent launch per call
-    shapes = solver.autotune(3) if not (args.no_autotune or whole) else solver.launch_shape()
-    # replay whole explicit_solve calls as CUDA graphs (no launch gaps between
-    # the passes; on small meshes launch latency dominates); the published case
-    # runs as one persistent launch per call (sequential LocalAccTime1)
+    # one resident launch per call (small meshes, the sequential time step), else passes
+    resident = bool(solver.schedule_info()["wavefront"])
+    shapes = solver.autotune(3) if not (args.no_autotune or resident) else solver.launch_shape()
+    # replay whole explicit_solve calls of passes as CUDA graphs (no launch gaps between them)
     if args.graphs == "on":
         solver.use_graphs(True)
 
@@ -561,8 +561,9 @@ def run_gpu(args):
 
     # warm-up
     solver.explicit_solve(args.warmup * per_step)
-    if solver.graphs_on and not whole:  # capture the timed call's graphs (one per buffer parity) outside the timed region
+    if not whole:  # buffers of the timed call's length outside the timed region
         solver.explicit_solve(args.steps * per_step)
+    if solver.graphs_on and not resident:  # and its graphs, one per buffer parity
         solver.explicit_solve(args.steps * per_step)
         solver.explicit_solve(per_step)
         solver.explicit_solve(per_step)
@@ -598,23 +599,26 @@ def run_gpu(args):
     clocks = clk.summary()
     ms_max, e2e_max = max_over_ranks([ms, e2e_s], ws, "cuda")
     value, e2e_value = replica_throughput(ws, nint * per_step, args.steps, ms_max, e2e_max)
-    # per-kernel timing for the roofline (CUDA events around each launch)
-    prof = solver.profile(2 * per_step if whole else 2)
+    # per-kernel timing for the roofline (CUDA events around each launch of the passes;
+    # the resident launch is the timed region itself)
+    prof = {"resident": (ms_max / args.steps / per_step * 2, 2)} if resident else solver.profile(2)
     nnz = 2 * grid.nface - grid.nghost  # CSR entries: interior faces twice, boundary faces once
     kernel, (kms, kcnt) = max(prof.items(), key=lambda kv: kv[1][0])
     peak, peak_kind = peaks()
     finite = bool(np.all(np.isfinite(linf))) and bool(np.all(np.isfinite(out)))
-    if whole:
+    if resident:
         info = solver.schedule_info()
-        nopi = sc.rk_level + (1 if sc.order == 2 else 0)
-        nsteps = info["period"] * (2 * per_step * nopi - 1) + info["levels"] + 1  # of the profiled call
-        roof = {"bound": "latency", "kernel": "wavefront", "achieved": None, "peak": peak, "peak_kind": peak_kind,
+        nops = args.steps * per_step * (sc.rk_level + (1 if sc.order == 2 else 0))
+        seq = sc.lc == 1 and sc.lc1_mode == 0
+        nsteps = info["period"] * (nops - 1) + info["levels"] if seq else nops
+        roof = {"bound": "latency", "kernel": "resident", "achieved": None, "peak": peak, "peak_kind": peak_kind,
                 "unit": "GB/s", "frac": None, "traffic": None,
-                "note": "one persistent launch per call; a %d-iteration call is %d steps of the level chain "
-                        "(period %d, %d levels, %d CTAs), %.2f us per step: bound by the exchange of states and "
-                        "a step's own instructions, not by HBM" %
-                        (2 * per_step, nsteps, info["period"], info["levels"], info["blocks"],
-                         1000.0 * kms / kcnt / nsteps)}
+                "note": "one persistent launch per call (several above 256 MB of norm rows); the timed call is a chain "
+                        "of %d %s (%d CTAs), %.2f us each: bound by the exchange of states between cells and an "
+                        "operation's own instructions, not by HBM" %
+                        (nsteps, "steps of the level chain (period %d, %d levels)" % (info["period"], info["levels"])
+                         if seq else "operations, a gradient or an RK stage of every cell", info["blocks"],
+                         1000.0 * ms_max / nsteps)}
     else:
         algo = traffic_model(grid, nnz, kernel, wl["precision"])
         achieved = algo / (kms / kcnt / 1000.0) / 1e9
@@ -654,8 +658,8 @@ def run_gpu(args):
                        "precision": ("FP32 state/flux; FP64 geometry, RK state, residual norms"
                                      if wl["precision"] == 32 else "FP64 throughout (the parity path)"),
                        "parallelism": "replicas" if ws > 1 else "single GPU",
-                       "threads_per_block": shapes,
-                       "cuda_graphs": args.graphs == "on" and not whole,
+                       "threads_per_block": {"resident": 128} if resident else shapes,
+                       "cuda_graphs": args.graphs == "on" and not resident,
                        "l2_flush": ("not needed: >2.5 GB of mesh + state per step, L2 is 126 MB" if wl["dim"] == 3
                                     else "none: this small case stays in L2 (not the bandwidth benchmark)")},
             "e2e": {"value": e2e_value, "unit": "cell-updates/s",
@@ -670,7 +674,7 @@ def run_gpu(args):
             "gpu_launches": int(launches),
             "clocks": clocks,
             "roofline": roof,
-            "kernel_ms_per_iteration": {k: v[0] / (2 * per_step if whole else 2) for k, v in prof.items()},
+            "kernel_ms_per_iteration": {k: v[0] / 2 for k, v in prof.items()},
             "library_device_ms": lib_ms,
             "finite": finite,
         }
