@@ -200,7 +200,11 @@ psst_status psst_grid_set_boundary(psst_grid *g, const char *zone_name, int dyn_
 /* ------------------------------------------------------------------------ */
 
 /* Uploads grid and scheme to `device`. Replaces the strategy construction and
- * initialize() calls in solver_parameters (psstFiniteVolumeGrid.cpp:50-192). */
+ * initialize() calls in solver_parameters (psstFiniteVolumeGrid.cpp:50-192).
+ * Device memory per face: the records (48 to 96 bytes by dimension and
+ * precision) and the columns that the face pass reads of them (20 to 88 bytes);
+ * where calls run resident, 0.6 to 2 KB a cell for that launch as well, and up to
+ * 0.7 KB more for sequential meshes of several work items a CTA. */
 psst_status psst_solver_create(const psst_grid *g, const psst_scheme *scheme, int device,
                                psst_solver **out);
 
@@ -285,7 +289,9 @@ psst_status psst_solver_profile(psst_solver *s, int n_iter, double *ms_per_kind,
  * so the next psst_explicit_solve continues from where it was. blocks (may be
  * NULL) receives the chosen shapes {gradient, face, cell}. The shapes change
  * no result except the last bits of the RMS column (its block partials follow
- * the cell-pass shape). Allocates a state-sized snapshot for the call. */
+ * the cell-pass shape). Allocates a state-sized snapshot for the call. A solver
+ * whose calls run as the resident launch (psst_solver_schedule_info) does not
+ * launch these passes: there is nothing to tune for it. */
 psst_status psst_solver_autotune(psst_solver *s, int n_iter, int *blocks);
 
 /* Sets (set != NULL; 0 keeps an entry) and/or reads (get != NULL) the launch

@@ -13,7 +13,6 @@ constexpr int kBlock = 256;
 constexpr int kMinBlock = 64;  // smallest launch shape the tuner may pick
 constexpr int kWfBlock = 128;  // threads per CTA of k_resident
 constexpr int kWfLanes = 4;    // lanes per cell in k_resident (cells per work item: 32)
-
 constexpr int kWfSyncWords = 96;  // k_resident's counter and flag words (three 128-byte lines)
 constexpr int kNormReduceBlocks = 296;  // most blocks a stage of k_norm_reduce (first level of its two-level sum)
 inline int nblocks(int64_t n, int b = kBlock) { return (int)((n + b - 1) / b); }
@@ -87,12 +86,12 @@ struct Ops {
     // the static face data of its items (FaceData), from the grid's arrays: mate
     // per CSR entry the same face's entry in the cell across, pos per cell its
     // place item * 32 + slot
-    // the face pass's columns: their size (FaceCols), and filling them from the face records
-    static size_t face_columns_bytes(int dim, int rec, int64_t nface);
-    static void face_columns(int dim, int rec, const DevGrid &g, char *cols, cudaStream_t s);
     static void resident_build(int dim, int rec, int grad, const DevGrid &g, const int32_t *cells32,
                                const uint32_t *lowmask, const int32_t *mate, const int32_t *pos, int nitems,
                                int rounds, void *faces, void *cells, cudaStream_t s);
+    // the face pass's columns: their size (FaceCols), and filling them from the face records
+    static size_t face_columns_bytes(int dim, int rec, int64_t nface);
+    static void face_columns(int dim, int rec, const DevGrid &g, char *cols, cudaStream_t s);
 };
 
 }  // namespace psst
