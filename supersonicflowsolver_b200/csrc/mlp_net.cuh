@@ -17,8 +17,8 @@
 // the instruction cache (24000 cycles instead of 11000 a backward layer).
 //
 // Measured, before -> now: training step of 16384 points, device 620 -> 112 us
-// (k_net 67, k_wgrad 30, k_reduce 15), call 650 -> 163 us; forward of 19200 points
-// (150 CTAs: two waves of 32 us) 409 -> 87 us. Every sum keeps the order of the
+// (k_net 67, k_wgrad 30, k_reduce 15), call 650 -> 150 to 163 us; forward of 19200 points
+// (150 CTAs: two waves of 32 us) 409 -> 88 us. Every sum keeps the order of the
 // layer-by-layer kernels it replaces, so the parameters are the same bits.
 #pragma once
 

@@ -40,12 +40,13 @@
 // lane. One lane a cell, four faces interleaved, was measured too: 3640
 // instructions an operation and twice the time.
 //
-// Measured (a whole call, set_state to norms, launch-by-launch or one-CTA-a-level
-// chain before -> now): 60 x 20 FP64, one iteration 155 -> 111 us; 120 x 40 FP64,
-// 100 iterations 5.25 -> 1.99 ms; 240 x 80 FP32, 50 iterations 2.11 -> 1.49 ms;
-// sequential 240 x 80 (first order, 300) 8.55 -> 4.16 ms and 120 x 40 (30) 4.15 -> 1.52 ms. An operation
-// of the 120 x 40 case takes some 8300 cycles: 900 for the static data, 900
-// waiting for neighbours, 2400 fluxes, 800 the sums over the faces, 1450 update and
+// Measured (a whole call, state in to state out, launch-by-launch or one-CTA-a-level
+// chain before -> now): 60 x 20 FP64, one iteration 155 -> 113 us; 120 x 40 FP64,
+// 100 iterations 5.23 -> 2.00 ms; 240 x 80 FP32, 50 iterations 2.11 -> 1.45 ms;
+// sequential 240 x 80 (first order, 300) 8.56 -> 4.16 ms and 120 x 40 (30) 4.16 -> 1.53
+// ms. An operation of the 120 x 40 case takes some 7900 cycles; of the 8300 that a copy
+// with clock64 in it took: 900 for the static data, 900 waiting for neighbours, 2400
+// fluxes, 800 the sums over the faces, 1450 update and
 // publication, 550 ghosts, 350 norms, 900 the loop and its barrier.
 //
 // Every wait is bounded: one longer than wait_ns sets the abort flag and

@@ -824,11 +824,14 @@ void build_resident(psst_solver *s) {
     }
     // The parallel modes: up to the sizes where it is the faster form. Every
     // interior face's flux is formed twice and a cell's faces take turns four at a
-    // time, against ten launches an iteration: us an iteration, resident / passes,
-    // HLLC MUSCL RK4: FP64 quads 4800 24.4 / 52.2, 10800 44.1 / 57.2, 19200 (two
-    // items a CTA) 72 / 65; FP32 quads 4800 17.9 / 38.9, 19200 33.4 / 44.5, 30000
-    // 58 / 46; with more than four faces a cell: FP64 hanging nodes 4906 55 / 64,
-    // 11298 126 / 67, hexes 2304 64.5 / 63.5; FP32 hexes 18432 46.8 / 57.8.
+    // time, against ten launches an iteration: us an iteration, resident / passes at
+    // their best shapes, HLLC MUSCL RK4: FP64 quads 4800 19.1 / 42.6, 13200 33.4 / 42.3,
+    // tets 6144 27.8 / 47.2; FP32 quads 4800 17.5 / 33.9, 19200 30.4 / 35.1, 22360 37.3 /
+    // 34.8, tets 15972 28.3 / 35.5, 20736 41.5 / 37.3 (the last sizes before the line
+    // lose a little); with more than four faces a cell: FP64 hanging nodes 4603 38.0 /
+    // 54.3; FP32 hanging nodes 10833 37.6 / 38.3, hexes 13552 36.9 / 45.0, 18432 45.5 /
+    // 45.1. Beyond it (both forms were slower then): FP64 quads 19200 (two items a CTA)
+    // 72 / 65, hanging nodes 11298 126 / 67, hexes 2304 64.5 / 63.5; FP32 quads 30000 58 / 46.
     if (!s->seq) {
         const bool f32 = sizeof(R) == 4, many = w.rounds > 1;
         if (f32 ? many && s->res_more : many && (s->dim == 3 || nitems > maxb / 2)) return;
