@@ -25,7 +25,8 @@ is involved.
           one process per host core, on a reduced mesh of the same workload
 
 --impl reference runs the reference's CPU implementation of the path on the
-host cores instead and prints the same metric.
+host cores instead and prints the same metric, or that it is unavailable where
+the reference was not there to be compiled.
 Multi-GPU: the path runs as independent replicas (one case per GPU, no
 collective); value = all ranks' cell-updates / max rank time.
 """
@@ -314,6 +315,10 @@ def cpu_baseline(warm, steps, workload):
 def run_reference_arm(args):
     ws, rank, _ = dist_env()
     if rank != 0:
+        return
+    if reference_binary()[1] != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not here to be compiled; "
+                                                              "its restatement in oracle/ is not the reference"}))
         return
     iters = WORKLOADS[args.workload].get("cpu_iters")
     warm, steps = (1, iters) if iters else (args.warmup, args.steps)
